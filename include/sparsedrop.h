@@ -324,6 +324,21 @@ int sd_gemm_sdd_relu_mask(const void* A, int64_t a_rs, int64_t a_cs,
                           const void* X, int64_t x_rs,
                           float scale, int dtype, void* workspace, int* status, void* stream);
 
+/* sd_gemm_sdd (X NULL) or sd_gemm_sdd_relu_mask with an fp32 result: the input gradient of an activation that is kept
+ * in fp32 (autocast), without the 16-bit tensor and the cast kernel autograd puts in between
+ * (flash_dropout/functional/blockwise_dropout_matmul_cuda.py:35-45 under autocast). */
+int sd_gemm_sdd_f32(const void* A, int64_t a_rs, int64_t a_cs,
+                    const void* B, int64_t b_rs, int64_t b_cs,
+                    float* C, int64_t c_rs, int64_t c_cs,
+                    int M, int N, int K, const void* plan,
+                    const void* X, int64_t x_rs,
+                    float scale, int dtype, void* workspace, int* status, void* stream);
+
+/* 16-bit copies (dtype SD_F16 or SD_BF16, round to nearest even) of one or two contiguous fp32 tensors from one launch:
+ * the casts of a layer's input and weight under autocast (blockwise_dropout_matmul_cuda.py:9).  A length may be 0;
+ * pointers must be 16-byte aligned. */
+int sd_cast16(const float* a, void* a16, int64_t na, const float* b, void* b16, int64_t nb, int dtype, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Fused convolution: im2col + DSD in one kernel.  The A operand of the product is the im2col matrix of
  * flash_dropout/functional/im2col_conv2d.py:17-20 (rows = output pixels m = (n, p, q), columns k = c*R*S + r*S + s),

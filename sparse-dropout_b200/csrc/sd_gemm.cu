@@ -151,7 +151,8 @@ struct GemmArgs {
     int a_panel_kg, c_panel_kg;      // > 0: A / C is the conv's im2col matrix stored in panels of 128 pixels, each panel
                                      // [kg][128] (kg a multiple of 64); the tensor map then describes [panels*kg][128]
     int split;                       // 1: equal unit ranges with fix-up (needs the workspace); 0: whole tiles
-    int tma_store;                   // result written by TMA from a swizzled staging buffer: 1 row-major, 2 column-major
+    int tma_store;                   // result written by TMA from a swizzled staging buffer: 16-bit 1 row-major, 2 column-
+                                     // major; fp32 3 column-major, 4 row-major
     float* ws_slots;
     int* ws_flags;
     const unsigned char* direct_mask;   // DSD launches in which a CTA gets only a few tiles: the plan's tile mask
@@ -545,7 +546,14 @@ __device__ __forceinline__ void zero_tile(const GemmArgs& g, bool vec_ok, bool v
     if (g.out_f32) {
         if (g.out_acc) return;                                   // adding nothing
         float* C32 = static_cast<float*>(g.C);
-        if (g.c_rs == 1) {
+        if (g.c_cs == 1 && (g.c_rs & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 && row0 + 128 <= g.MM &&
+            col0 + 128 <= g.NN) {
+            const int cchunk = tid & 31, rsub = tid >> 5;        // a warp covers one 512-byte row of the tile
+#pragma unroll 4
+            for (int i = 0; i < 32; ++i)
+                *reinterpret_cast<float4*>(C32 + (long long)(row0 + i * 4 + rsub) * g.c_rs + col0 + cchunk * 4) =
+                    make_float4(0.f, 0.f, 0.f, 0.f);
+        } else if (g.c_rs == 1) {
             for (int j = 0; j < 128; ++j)
                 if (row0 + tid < g.MM && col0 + j < g.NN) C32[(long long)(col0 + j) * g.c_cs + row0 + tid] = 0.f;
         } else {
@@ -674,6 +682,10 @@ __device__ bool reduce_shared_tile(const GemmArgs& g, const Seg& seg, int eidx, 
         }
         if (g.out_f32) {
             float* C32 = static_cast<float*>(g.C);
+            if (!g.out_acc && g.c_cs == 1 && (g.c_rs & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0 && col + 4 <= g.NN) {
+                *reinterpret_cast<float4*>(C32 + (long long)row * g.c_rs + col) = make_float4(f[0], f[1], f[2], f[3]);
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 if (col + j < g.NN) {
@@ -1191,6 +1203,25 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
                         bulk_commit();
                     }
                     ++n_stores;
+                } else if (g.tma_store == 4) {
+                    // fp32 row-major result (an input gradient for an fp32 activation): one chunk = 32 rows of 128
+                    // bytes, 16-byte pieces XOR-swizzled (CU_TENSOR_MAP_SWIZZLE_128B), one TMA store
+                    const uint32_t buf = stage_base + (two_bufs ? ((n_stores & 1) << 12) : 0);
+                    wait_staging_free(two_bufs, n_stores, lane);
+                    const uint32_t rowaddr = buf + lane * 128, sw = lane & 7;
+#pragma unroll
+                    for (int v = 0; v < 8; ++v)
+                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + ((v ^ sw) << 4)),
+                                     "f"(__uint_as_float(r[4 * v]) * g.scale), "f"(__uint_as_float(r[4 * v + 1]) * g.scale),
+                                     "f"(__uint_as_float(r[4 * v + 2]) * g.scale), "f"(__uint_as_float(r[4 * v + 3]) * g.scale)
+                                     : "memory");
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_2d(&tmapC, buf, col, w.a_row + quad * 32);
+                        bulk_commit();
+                    }
+                    ++n_stores;
                 } else if (g.out_f32) {
                     store_chunk_f32(g, row, col, r);
                 } else {
@@ -1560,8 +1591,8 @@ static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const v
     // Row-major result with 16-byte rows: written by TMA (clipped at the ragged edge); otherwise by the warps.
     CUtensorMap tc = ta;
     if (g.out_f32) {
-        // an fp32 result that overwrites a column-major matrix with 16-byte aligned columns leaves by TMA; other
-        // fp32 results (row-major, accumulating, unaligned) are written by the epilogue warps directly
+        // an fp32 result that overwrites a matrix with 16-byte aligned columns (or rows) leaves by TMA; other
+        // fp32 results (accumulating, unaligned) are written by the epilogue warps directly
         if (!g.out_acc && c_rs == 1 && (c_cs & 3) == 0 && c_cs >= M && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
             EncodeTiledFn enc = encode_tiled_fn();
             cuuint64_t dims[2] = {cuuint64_t(M), cuuint64_t(N)};            // the transpose, row-major [N][M]
@@ -1573,6 +1604,17 @@ static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const v
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(fp32 C^T) failed with CUresult %d", int(r));
             g.tma_store = 3;
+        } else if (!g.out_acc && c_cs == 1 && (c_rs & 3) == 0 && c_rs >= N && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+            EncodeTiledFn enc = encode_tiled_fn();
+            cuuint64_t dims[2] = {cuuint64_t(N), cuuint64_t(M)};
+            cuuint64_t strides[1] = {cuuint64_t(M > 1 ? c_rs * 4 : ((int64_t(N) * 4 + 15) & ~int64_t(15)))};
+            cuuint32_t box[2] = {32u, 32u};
+            cuuint32_t estr[2] = {1u, 1u};
+            CUresult r = enc(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(fp32 C) failed with CUresult %d", int(r));
+            g.tma_store = 4;
         }
     } else if (c_panel_kg) {
         EncodeTiledFn enc = encode_tiled_fn();
@@ -1798,6 +1840,17 @@ int sd_gemm_sdd_relu_mask(const void* A, int64_t a_rs, int64_t a_cs, const void*
                           float scale, int dtype, void* workspace, int* status, void* stream) {
     if (!X) return sd::fail(SD_ERR_INVALID_ARG, "X is null");
     sd::GemmExtras ex;
+    ex.mask_src = X;
+    ex.mask_rs = x_rs;
+    return sd::run_gemm(sd::MODE_SDD, A, a_rs, a_cs, B, b_rs, b_cs, C, c_rs, c_cs, M, N, K, plan, 0, scale, dtype,
+                        workspace, status, stream, 0, true, false, 0, nullptr, 0, &ex);
+}
+
+int sd_gemm_sdd_f32(const void* A, int64_t a_rs, int64_t a_cs, const void* B, int64_t b_rs, int64_t b_cs, float* C,
+                    int64_t c_rs, int64_t c_cs, int M, int N, int K, const void* plan, const void* X, int64_t x_rs,
+                    float scale, int dtype, void* workspace, int* status, void* stream) {
+    sd::GemmExtras ex;
+    ex.out_f32 = 1;
     ex.mask_src = X;
     ex.mask_rs = x_rs;
     return sd::run_gemm(sd::MODE_SDD, A, a_rs, a_cs, B, b_rs, b_cs, C, c_rs, c_cs, M, N, K, plan, 0, scale, dtype,

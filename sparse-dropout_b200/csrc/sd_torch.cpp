@@ -1,0 +1,600 @@
+// The operator API's path from torch tensors to libsparsedrop.so, in native code: argument checks, the casts under
+// autocast, the mask draw, the launches and the autograd nodes of a SparseDrop linear and of the LayerNorm in front of it.
+//
+// A small layer is bound by the host: its four kernels take 31 us at 512^3 while the same sequence issued from Python
+// (ctypes calls, a Python autograd.Function, tensor bookkeeping) took 197 us per forward + backward.  Everything between
+// the Python entry points and the C ABI therefore runs here; the C-ABI library itself stays free of torch.
+//
+// Replaces the glue of flash_dropout/functional/blockwise_dropout_matmul_cuda.py:7-59 and
+// flash_dropout/cuda/src/gemm_binding.cu:44-141.
+#include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_cpp_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <mutex>
+#include <optional>
+#include <unordered_map>
+#include <vector>
+
+#include "../../include/sparsedrop.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+constexpr int TILE = 128;
+inline int64_t tiles_of(int64_t n) { return (n + TILE - 1) / TILE; }
+
+// Raised as flash_dropout._lib.SparseDropError (a RuntimeError).
+struct SdError : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+inline void check_rc(int rc) {
+    if (rc != 0) throw SdError("libsparsedrop error " + std::to_string(rc) + ": " + sd_last_error());
+}
+[[noreturn]] inline void bad(const std::string& msg) { throw std::runtime_error(msg); }
+
+int dtype_code(at::ScalarType t) {
+    if (t == at::kHalf) return SD_F16;
+    if (t == at::kBFloat16) return SD_BF16;
+    throw SdError(std::string("operands must be half or bfloat16, got ") + c10::toString(t));
+}
+
+inline Tensor empty2(int64_t a, int64_t b, at::ScalarType t, const at::Device& d) {
+    return at::detail::empty_cuda({a, b}, t, d, std::nullopt);
+}
+inline Tensor empty_bytes(int64_t n, const at::Device& d) { return at::detail::empty_cuda({n}, at::kByte, d, std::nullopt); }
+
+// ---------------------------------------------------------------- per-device state
+// The failure-detection words and the split-schedule workspaces, one per (device, stream) that has launched products:
+// launches that can overlap on the GPU must not share a workspace.  Lives until the process exits.
+struct DeviceState {
+    Tensor status;
+    std::unordered_map<cudaStream_t, Tensor> workspaces;
+};
+std::mutex& state_mutex() { static auto* m = new std::mutex; return *m; }
+std::unordered_map<int, DeviceState>& states() { static auto* s = new std::unordered_map<int, DeviceState>; return *s; }
+
+Tensor status_tensor(int dev) {
+    std::lock_guard<std::mutex> lock(state_mutex());
+    DeviceState& s = states()[dev];
+    if (!s.status.defined())
+        s.status = at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, c10::DeviceIndex(dev))));
+    return s.status;
+}
+Tensor workspace_tensor(int dev, cudaStream_t stream) {
+    std::lock_guard<std::mutex> lock(state_mutex());
+    Tensor& ws = states()[dev].workspaces[stream];
+    if (!ws.defined()) {
+        const at::Device d(at::kCUDA, c10::DeviceIndex(dev));
+        c10::cuda::CUDAGuard guard(d);
+        Tensor t = empty_bytes(int64_t(sd_workspace_bytes()), d);
+        check_rc(sd_workspace_init(t.data_ptr(), stream));
+        ws = t;
+    }
+    return ws;
+}
+
+// What every launch needs besides its operands.  The two pointers are looked up once per thread, device and stream.
+struct Launch {
+    cudaStream_t stream;
+    int* status;
+    void* ws;
+    explicit Launch(const at::Device& d) {
+        struct Cached { int dev = -1; cudaStream_t stream = nullptr; int* status = nullptr; void* ws = nullptr; };
+        static thread_local Cached c;
+        stream = c10::cuda::getCurrentCUDAStream(d.index()).stream();
+        if (c.dev != d.index() || c.stream != stream) {
+            c.status = status_tensor(d.index()).data_ptr<int>();
+            c.ws = workspace_tensor(d.index(), stream).data_ptr();
+            c.dev = d.index();
+            c.stream = stream;
+        }
+        status = c.status;
+        ws = c.ws;
+    }
+};
+
+struct Mat { void* p; int64_t rs, cs; };
+inline Mat mat(const Tensor& t) { return {t.data_ptr(), t.stride(0), t.stride(1)}; }
+inline Mat mat_t(const Tensor& t) { return {t.data_ptr(), t.stride(1), t.stride(0)}; }
+
+// Row- or column-major with a TMA-compatible leading stride, else a contiguous copy.
+Tensor operand(const Tensor& x) {
+    if (reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0) {
+        const int64_t r = x.size(0), c = x.size(1), sr = x.stride(0), sc = x.stride(1);
+        if (sc == 1 && (sr % 8 == 0 || r == 1) && sr >= c) return x;
+        if (sr == 1 && (sc % 8 == 0 || c == 1) && sc >= r) return x;
+    }
+    Tensor y = x.contiguous();
+    // a contiguous view that starts off a 16-byte boundary is copied as well
+    return reinterpret_cast<uintptr_t>(y.data_ptr()) % 16 == 0 ? y : y.clone();
+}
+
+// ---------------------------------------------------------------- block plans
+// How the mask of one call comes about: a plan that exists, or a draw from (seed, offset), the offset optionally
+// advanced by a counter in device memory.
+struct Draw {
+    uint64_t seed = 0, offset = 0;
+    uint64_t* counter = nullptr;
+    int rep_r = 1, rep_c = 1;
+    float p = 0;
+};
+Tensor draw_plan(const Draw& d, int64_t M, int64_t K, const at::Device& dev, cudaStream_t stream) {
+    const int R = int(tiles_of(M)), C = int(tiles_of(K));
+    Tensor buf = empty_bytes(int64_t(sd_plan_bytes(R, C)), dev);
+    if (d.counter)
+        check_rc(sd_plan_from_seed_counter(buf.data_ptr(), R, C, d.rep_r, d.rep_c, d.seed, d.offset, d.counter, d.p, nullptr, stream));
+    else
+        check_rc(sd_plan_from_seed(buf.data_ptr(), R, C, d.rep_r, d.rep_c, d.seed, d.offset, d.p, nullptr, stream));
+    return buf;
+}
+
+// ---------------------------------------------------------------- casts under autocast
+inline bool flat_f32(const Tensor& t) {
+    return t.scalar_type() == at::kFloat && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+}
+
+// 16-bit copies of a and, if given, b: one launch where both are contiguous fp32.
+void cast_pair(const Tensor& a, Tensor& a16, const Tensor& b, Tensor& b16, at::ScalarType dt, cudaStream_t stream) {
+    const bool fa = a.defined() && flat_f32(a), fb = b.defined() && flat_f32(b);
+    if (a.defined()) a16 = fa ? Tensor(at::detail::empty_cuda(a.sizes(), dt, a.device(), std::nullopt)) : a.to(dt);
+    if (b.defined()) b16 = fb ? Tensor(at::detail::empty_cuda(b.sizes(), dt, b.device(), std::nullopt)) : b.to(dt);
+    if (fa || fb)
+        check_rc(sd_cast16(fa ? a.data_ptr<float>() : nullptr, fa ? a16.data_ptr() : nullptr, fa ? a.numel() : 0,
+                           fb ? b.data_ptr<float>() : nullptr, fb ? b16.data_ptr() : nullptr, fb ? b.numel() : 0,
+                           dtype_code(dt), stream));
+}
+
+// The copy of the last activation this thread cast, for consecutive layers that are fed the very same tensor (the q / k / v
+// projections of an attention block).  A layer sees a fresh 2-D view on every call, so the tensor is identified by the one
+// that owns its memory plus the view's geometry and version; only weak references are held, so an entry dies with its
+// tensor and keeps no memory alive.
+struct CastEntry {
+    c10::weak_intrusive_ptr<c10::TensorImpl> owner, copy;
+    uint32_t version;
+    at::ScalarType dt;
+    int64_t offset, size[2], stride[2];
+    cudaStream_t stream;
+};
+struct CastCache {
+    std::optional<CastEntry> e;
+    static Tensor owner_of(const Tensor& x) { return x.is_view() ? Tensor(x._base()) : x; }
+    Tensor find(const Tensor& x, at::ScalarType dt, cudaStream_t stream) {
+        if (!e || x.is_inference() || e->dt != dt || e->stream != stream || e->version != x._version() || e->offset != x.storage_offset()) return {};
+        for (int i = 0; i < 2; ++i)
+            if (e->size[i] != x.size(i) || e->stride[i] != x.stride(i)) return {};
+        auto own = e->owner.lock();
+        if (!own || own.get() != owner_of(x).unsafeGetTensorImpl()) return {};
+        auto copy = e->copy.lock();
+        return copy ? Tensor(std::move(copy)) : Tensor();
+    }
+    void put(const Tensor& x, const Tensor& x16, cudaStream_t stream) {
+        if (x.is_inference()) return;
+        e.emplace(CastEntry{c10::weak_intrusive_ptr<c10::TensorImpl>(owner_of(x).getIntrusivePtr()),
+                            c10::weak_intrusive_ptr<c10::TensorImpl>(x16.getIntrusivePtr()), uint32_t(x._version()), x16.scalar_type(),
+                            x.storage_offset(), {x.size(0), x.size(1)}, {x.stride(0), x.stride(1)}, stream});
+    }
+};
+
+// ---------------------------------------------------------------- a SparseDrop linear
+struct PyCallback {
+    PyObject* f;
+    explicit PyCallback(PyObject* f_) : f(f_) { Py_INCREF(f); }
+    PyCallback(const PyCallback&) = delete;
+    ~PyCallback() {
+        if (Py_IsInitialized()) {
+            py::gil_scoped_acquire gil;
+            Py_DECREF(f);
+        }
+    }
+    void operator()() const {
+        py::gil_scoped_acquire gil;
+        PyObject* r = PyObject_CallNoArgs(f);
+        if (!r) throw py::error_already_set();
+        Py_DECREF(r);
+    }
+};
+
+struct Options {
+    bool relu = false, input_relu = false, premasked = false;
+    Tensor wgrad;                                  // fp32 [out, in]: the weight gradient goes straight there
+    bool wgrad_acc = false;
+    std::shared_ptr<PyCallback> notify;
+};
+
+struct SparseDropLinearBackward : public Node {
+    SavedVariable x, w, y;                         // 16-bit operands of the forward product; y: its ReLU'd result
+    Tensor plan;                                   // undefined: drawn again from `draw` (recompute_plan)
+    Draw draw;
+    int64_t block_m = 0, block_k = 0;
+    bool pair_block = false;
+    int64_t M = 0, K = 0, N = 0;
+    double p = 0;
+    bool x_f32 = false, w_f32 = false;             // the layer's own tensors are fp32: their gradients leave in fp32
+    Options opt;
+
+    std::string name() const override { return "SparseDropLinearBackward"; }
+    void release_variables() override {
+        x.reset_data();
+        w.reset_data();
+        y.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override;
+};
+
+variable_list SparseDropLinearBackward::apply(variable_list&& grads) {
+    at::NoGradGuard no_grad;
+    const Tensor x16 = x.unpack(), w16 = w.unpack();
+    const at::Device dev = x16.device();
+    c10::cuda::OptionalCUDAGuard guard(dev);
+    const Launch L(dev);
+    const float scale = float(1.0 / (1.0 - p));
+    const int dt = dtype_code(x16.scalar_type());
+    const Tensor pl = plan.defined() ? plan : draw_plan(draw, M, K, dev, L.stream);
+    Tensor dy = grads[0].defined() ? grads[0] : at::zeros({M, N}, x16.options());
+    if (dy.scalar_type() != x16.scalar_type()) dy = dy.to(x16.scalar_type());
+    if (opt.relu && !opt.premasked) dy = at::threshold_backward(dy, y.unpack(shared_from_this()), 0);
+    dy = operand(dy);
+    const Mat mdy = mat(dy), mx = mat(x16), mdyt = mat_t(dy), mxt = mat_t(x16), mwt = mat_t(w16);
+    Tensor dx, dw;
+    if (task_should_compute_output(0)) {
+        // dx (M, K) = keep o (dy (M, N) . W (N, K)) * scale
+        dx = empty2(M, K, x_f32 ? at::kFloat : x16.scalar_type(), dev);
+        void* mask = opt.input_relu ? mx.p : nullptr;
+        if (x_f32)
+            check_rc(sd_gemm_sdd_f32(mdy.p, mdy.rs, mdy.cs, mwt.p, mwt.rs, mwt.cs, dx.data_ptr<float>(), K, 1, int(M), int(K), int(N),
+                                     pl.data_ptr(), mask, mx.rs, scale, dt, L.ws, L.status, L.stream));
+        else if (mask)
+            check_rc(sd_gemm_sdd_relu_mask(mdy.p, mdy.rs, mdy.cs, mwt.p, mwt.rs, mwt.cs, dx.data_ptr(), K, 1, int(M), int(K), int(N),
+                                           pl.data_ptr(), mask, mx.rs, scale, dt, L.ws, L.status, L.stream));
+        else
+            check_rc(sd_gemm_sdd(mdy.p, mdy.rs, mdy.cs, mwt.p, mwt.rs, mwt.cs, dx.data_ptr(), K, 1, int(M), int(K), int(N),
+                                 pl.data_ptr(), scale, dt, L.ws, L.status, L.stream));
+    }
+    // dW^T (K, N) = (keep o x)^T (K, M) . dy (M, N) * scale, stored straight into dW (N, K)
+    if (opt.wgrad.defined()) {
+        check_rc(sd_gemm_dsd_f32(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, opt.wgrad.data_ptr<float>(), opt.wgrad.stride(1),
+                                 opt.wgrad.stride(0), int(K), int(N), int(M), pl.data_ptr(), SD_PLAN_COLS, scale, dt,
+                                 int(opt.wgrad_acc), L.ws, L.status, L.stream));
+        if (opt.notify) (*opt.notify)();
+    } else if (task_should_compute_output(1)) {
+        dw = empty2(N, K, w_f32 ? at::kFloat : w16.scalar_type(), dev);
+        if (w_f32)
+            check_rc(sd_gemm_dsd_f32(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, dw.data_ptr<float>(), 1, K, int(K), int(N), int(M),
+                                     pl.data_ptr(), SD_PLAN_COLS, scale, dt, 0, L.ws, L.status, L.stream));
+        else
+            check_rc(sd_gemm_dsd(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, dw.data_ptr(), 1, K, int(K), int(N), int(M),
+                                 pl.data_ptr(), SD_PLAN_COLS, scale, dt, L.ws, L.status, L.stream));
+    }
+    return {dx, dw};
+}
+
+// y = (keep o input) . weight^T / (1 - p) of 2-D CUDA tensors, see blockwise_dropout_matmul in
+// functional/blockwise_dropout_matmul_cuda.py for the meaning of the arguments.  `plan` with its grid, or none: drawn from
+// (seed, offset) and the optional device counter.  `recompute`: (seed, offset) are all that is kept for backward.
+Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<Tensor>& plan_, int64_t plan_R, int64_t plan_C,
+              int64_t rep_r, int64_t rep_c, bool pair_block, double p, uint64_t seed, uint64_t offset,
+              const std::optional<Tensor>& counter, bool relu, bool input_relu, bool premasked,
+              const std::optional<Tensor>& wgrad, bool wgrad_acc, py::handle notify, bool recompute,
+              const std::optional<Tensor>& weight_lowp) {
+    Options opt;
+    opt.relu = relu;
+    opt.input_relu = input_relu;
+    opt.premasked = premasked;
+    if (wgrad && wgrad->defined()) {
+        opt.wgrad = *wgrad;
+        opt.wgrad_acc = wgrad_acc;
+        if (!notify.is_none()) opt.notify = std::make_shared<PyCallback>(notify.ptr());
+    }
+    py::gil_scoped_release no_gil;
+    if (!input_.is_cuda() || !weight_.is_cuda()) bad("input and weight must be CUDA");   // no CPU path, as gemm_binding.cu:19
+    if (input_.dim() != 2 || weight_.dim() != 2) bad("input and weight must be 2D");
+    if (input_.device() != weight_.device()) bad("A and B must be on the same device");
+    const at::Device dev = input_.device();
+    c10::cuda::OptionalCUDAGuard guard(dev);
+    const Launch L(dev);
+
+    // operands in 16 bits; fp32 ones are cast here, outside autograd, and their gradients leave in fp32
+    Tensor input = input_, weight = weight_, x16, w16;
+    if (at::autocast::is_autocast_enabled(at::kCUDA)) {
+        const at::ScalarType dt = at::autocast::get_autocast_dtype(at::kCUDA);
+        const bool lowp = weight_lowp && opt.wgrad.defined() && weight_lowp->scalar_type() == dt && weight_lowp->sizes() == weight.sizes();
+        if (input.scalar_type() != dt && input.scalar_type() != at::kFloat) input = input.to(dt);
+        if (!lowp && weight.scalar_type() != dt && weight.scalar_type() != at::kFloat) weight = weight.to(dt);
+        at::NoGradGuard no_grad;
+        static thread_local CastCache cache;
+        const bool cast_x = input.scalar_type() != dt, cast_w = !lowp && weight.scalar_type() != dt;
+        x16 = input;
+        w16 = lowp ? *weight_lowp : weight;
+        if (cast_x) x16 = cache.find(input, dt, L.stream);
+        const bool hit = x16.defined();
+        if (!hit || cast_w) cast_pair(hit ? Tensor() : input, x16, cast_w ? weight : Tensor(), w16, dt, L.stream);
+        if (!hit) cache.put(input, x16, L.stream);
+    } else {
+        x16 = input;
+        w16 = weight;
+    }
+    if (x16.scalar_type() != w16.scalar_type())
+        bad(std::string("input (") + c10::toString(x16.scalar_type()) + ") and weight (" + c10::toString(w16.scalar_type()) +
+            ") must have the same dtype");
+    const int dt = dtype_code(x16.scalar_type());
+    const int64_t M = x16.size(0), K = x16.size(1), N = w16.size(0);
+    if (K % 8 || N % 8) bad("in_features and out_features must be multiples of 8 (16-byte TMA rows)");
+    if (w16.size(1) != K)
+        bad("reduction dimensions differ: A is (" + std::to_string(M) + ", " + std::to_string(K) + "), B is (" + std::to_string(N) +
+            ", " + std::to_string(w16.size(1)) + ")");
+    if (opt.wgrad.defined()) {
+        const Tensor& t = opt.wgrad;
+        if (t.dim() != 2 || t.size(0) != N || t.size(1) != K || t.device() != dev || t.scalar_type() != at::kFloat ||
+            !(t.stride(0) == 1 || t.stride(1) == 1))
+            bad("out has the wrong shape, device or strides");
+    }
+    const bool needs_grad = torch::autograd::compute_requires_grad(input, weight);
+    Tensor xs, ws, out, plan;
+    Draw d;
+    {
+        at::NoGradGuard no_grad;
+        xs = operand(x16);
+        ws = operand(w16);
+        if (input_relu && xs.stride(1) != 1) xs = xs.contiguous();
+        if (plan_ && plan_->defined()) {
+            if (plan_R != tiles_of(M) || plan_C != tiles_of(K))
+                bad("plan grid (" + std::to_string(plan_R) + ", " + std::to_string(plan_C) + ") does not match operand A (" +
+                    std::to_string(M) + ", " + std::to_string(K) + ")");
+            plan = *plan_;
+        }
+        d.seed = seed;
+        d.offset = offset;
+        d.counter = counter && counter->defined() ? static_cast<uint64_t*>(counter->data_ptr()) : nullptr;
+        d.rep_r = int(rep_r);
+        d.rep_c = int(rep_c);
+        d.p = float(p);
+        if (!plan.defined()) plan = draw_plan(d, M, K, dev, L.stream);
+        out = empty2(M, N, xs.scalar_type(), dev);
+        const Mat a = mat(xs), b = mat(ws);
+        check_rc((relu ? sd_gemm_dsd_relu : sd_gemm_dsd)(a.p, a.rs, a.cs, b.p, b.rs, b.cs, out.data_ptr(), N, 1, int(M), int(N), int(K),
+                                                         plan.data_ptr(), SD_PLAN_ROWS, float(1.0 / (1.0 - p)), dt, L.ws, L.status,
+                                                         L.stream));
+    }
+    if (!needs_grad) return out;
+    std::shared_ptr<SparseDropLinearBackward> node(new SparseDropLinearBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(input, weight));
+    node->x = SavedVariable(xs.is_same(x16) && x16.is_same(input) ? input : xs, false);
+    node->w = SavedVariable(ws.is_same(w16) && w16.is_same(weight) ? weight : ws, false);
+    node->draw = d;
+    node->block_m = rep_r * TILE;
+    node->block_k = rep_c * TILE;
+    node->pair_block = pair_block;
+    if (!recompute || d.counter) node->plan = plan;
+    node->M = M;
+    node->K = K;
+    node->N = N;
+    node->p = p;
+    node->x_f32 = input.scalar_type() == at::kFloat;
+    node->w_f32 = weight.scalar_type() == at::kFloat;
+    node->opt = std::move(opt);
+    torch::autograd::set_history(out, node);
+    if (relu && !premasked) node->y = SavedVariable(out, true);
+    return out;
+}
+
+// Python attributes of the node: the mask it holds (`plan`: the plan buffer, or None when it is drawn again in backward)
+// and what it is drawn from (`origin`: rows, columns, block size, p, seed, offset).
+SparseDropLinearBackward* node_of(PyObject* self) {
+    return static_cast<SparseDropLinearBackward*>(reinterpret_cast<torch::autograd::THPCppFunction*>(self)->cdata.get());
+}
+PyObject* get_plan(PyObject* self, void*) {
+    const auto* n = node_of(self);
+    if (!n->plan.defined()) Py_RETURN_NONE;
+    return THPVariable_Wrap(n->plan);
+}
+PyObject* get_origin(PyObject* self, void*) {
+    const auto* n = node_of(self);
+    if (n->plan.defined()) Py_RETURN_NONE;
+    py::object block = n->pair_block ? py::object(py::make_tuple(n->block_m, n->block_k)) : py::object(py::int_(n->block_m));
+    return py::make_tuple(n->M, n->K, block, n->p, n->draw.seed, n->draw.offset).release().ptr();
+}
+void register_node() {
+    using namespace torch::autograd;
+    static PyGetSetDef properties[] = {THP_FUNCTION_DEFAULT_PROPERTIES,
+                                       {(char*)"plan", get_plan, nullptr, nullptr, nullptr},
+                                       {(char*)"origin", get_origin, nullptr, nullptr, nullptr},
+                                       {nullptr}};
+    static PyTypeObject type;
+    _initFunctionPyTypeObject(type, "SparseDropLinearBackward", properties, nullptr);
+    Py_INCREF(&type);
+    registerCppFunction(typeid(SparseDropLinearBackward), &type);
+}
+
+// ---------------------------------------------------------------- the extension-style products
+std::string shape_text(int64_t a, int64_t b) { return "(" + std::to_string(a) + ", " + std::to_string(b) + ")"; }
+void check_operand(const Tensor& x, const char* name) {      // flash_dropout/cuda/src/gemm_binding.cu:18-22
+    if (!x.is_cuda()) bad(std::string(name) + " must be CUDA");
+    if (x.dim() != 2) bad(std::string(name) + " must be 2D");
+    if (!(x.stride(0) == 1 || x.stride(1) == 1)) bad(std::string(name) + " must be row or column major");
+}
+int check_pair(const Tensor& A, const Tensor& B) {
+    check_operand(A, "A");
+    check_operand(B, "B");
+    if (A.scalar_type() != B.scalar_type()) bad("A and B must have the same dtype");
+    if (A.size(1) != B.size(1))
+        bad("reduction dimensions differ: A is " + shape_text(A.size(0), A.size(1)) + ", B is " + shape_text(B.size(0), B.size(1)));
+    if (A.device() != B.device()) bad("A and B must be on the same device");
+    return dtype_code(A.scalar_type());
+}
+Tensor plan_from_mask(const Tensor& mask, int64_t rows, int64_t cols, int64_t rep_r, int64_t rep_c, cudaStream_t stream) {
+    if (mask.scalar_type() != at::kBool) bad("Mask must be bool");
+    if (!mask.is_cuda() || mask.dim() != 2) bad("Mask must be a 2D CUDA tensor");
+    const int64_t R = tiles_of(rows), C = tiles_of(cols), wr = (R + rep_r - 1) / rep_r, wc = (C + rep_c - 1) / rep_c;
+    if (mask.size(0) != wr || mask.size(1) != wc)
+        bad("mask shape " + shape_text(mask.size(0), mask.size(1)) + " does not match " + shape_text(wr, wc) + " blocks of " +
+            shape_text(rep_r * TILE, rep_c * TILE));
+    Tensor buf = empty_bytes(int64_t(sd_plan_bytes(int(R), int(C))), mask.device());
+    check_rc(sd_plan_from_mask(buf.data_ptr(), int(R), int(C), int(rep_r), int(rep_c), static_cast<const uint8_t*>(mask.data_ptr()),
+                               mask.stride(0), mask.stride(1), stream));
+    return buf;
+}
+
+Tensor gemm_dense(const Tensor& A, const Tensor& B) {
+    py::gil_scoped_release no_gil;
+    at::NoGradGuard no_grad;
+    const int dt = check_pair(A, B);
+    c10::cuda::OptionalCUDAGuard guard(A.device());
+    const Launch L(A.device());
+    Tensor C = empty2(A.size(0), B.size(0), A.scalar_type(), A.device());
+    const Mat a = mat(A), b = mat(B);
+    check_rc(sd_gemm(a.p, a.rs, a.cs, b.p, b.rs, b.cs, C.data_ptr(), C.size(1), 1, int(A.size(0)), int(B.size(0)), int(A.size(1)), 1.0f,
+                     dt, L.ws, L.status, L.stream));
+    return C;
+}
+Tensor gemm_dsd(const Tensor& A, const Tensor& B, const Tensor& mask, int64_t rep_r, int64_t rep_c, double scale) {
+    py::gil_scoped_release no_gil;
+    at::NoGradGuard no_grad;
+    check_operand(A, "A");
+    c10::cuda::OptionalCUDAGuard guard(A.device());
+    const Launch L(A.device());
+    const Tensor plan = plan_from_mask(mask, A.size(0), A.size(1), rep_r, rep_c, L.stream);
+    const int dt = check_pair(A, B);
+    Tensor C = empty2(A.size(0), B.size(0), A.scalar_type(), A.device());
+    const Mat a = mat(A), b = mat(B);
+    check_rc(sd_gemm_dsd(a.p, a.rs, a.cs, b.p, b.rs, b.cs, C.data_ptr(), C.size(1), 1, int(A.size(0)), int(B.size(0)), int(A.size(1)),
+                         plan.data_ptr(), SD_PLAN_ROWS, float(scale), dt, L.ws, L.status, L.stream));
+    return C;
+}
+Tensor gemm_sdd(const Tensor& A, const Tensor& B, const Tensor& mask, int64_t rep_r, int64_t rep_c, double scale) {
+    py::gil_scoped_release no_gil;
+    at::NoGradGuard no_grad;
+    check_operand(A, "A");
+    check_operand(B, "B");
+    c10::cuda::OptionalCUDAGuard guard(A.device());
+    const Launch L(A.device());
+    const Tensor plan = plan_from_mask(mask, A.size(0), B.size(0), rep_r, rep_c, L.stream);
+    const int dt = check_pair(A, B);
+    Tensor C = empty2(A.size(0), B.size(0), A.scalar_type(), A.device());
+    const Mat a = mat(A), b = mat(B);
+    check_rc(sd_gemm_sdd(a.p, a.rs, a.cs, b.p, b.rs, b.cs, C.data_ptr(), C.size(1), 1, int(A.size(0)), int(B.size(0)), int(A.size(1)),
+                         plan.data_ptr(), float(scale), dt, L.ws, L.status, L.stream));
+    return C;
+}
+
+// ---------------------------------------------------------------- LayerNorm
+int norm_code(at::ScalarType t) { return t == at::kHalf ? SD_F16 : t == at::kBFloat16 ? SD_BF16 : SD_F32; }
+
+struct SparseDropLayerNormBackward : public Node {
+    SavedVariable x, weight;
+    Tensor mean, rstd;
+    bool has_bias = false;
+    std::vector<int64_t> shape;
+
+    std::string name() const override { return "SparseDropLayerNormBackward"; }
+    void release_variables() override {
+        x.reset_data();
+        weight.reset_data();
+        mean.reset();
+        rstd.reset();
+    }
+    variable_list apply(variable_list&& grads) override {
+        at::NoGradGuard no_grad;
+        const Tensor x2 = x.unpack(), g = weight.unpack();
+        const at::Device dev = x2.device();
+        c10::cuda::OptionalCUDAGuard guard(dev);
+        cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+        const int64_t n = shape.back(), rows = x2.numel() / n;
+        Tensor dy = grads[0].defined() ? grads[0] : at::zeros(shape, x2.options());
+        const at::ScalarType t = dy.scalar_type();
+        if (t != at::kFloat && t != at::kHalf && t != at::kBFloat16) dy = dy.to(at::kFloat);
+        dy = dy.contiguous();
+        Tensor dx = at::detail::empty_cuda(shape, at::kFloat, dev, std::nullopt);
+        Tensor dg = at::detail::empty_cuda({n}, at::kFloat, dev, std::nullopt), db;
+        if (has_bias) db = at::detail::empty_cuda({n}, at::kFloat, dev, std::nullopt);
+        Tensor ws = empty_bytes(int64_t(sd_layernorm_bwd_workspace_bytes(int(rows), int(n))), dev);
+        check_rc(sd_layernorm_bwd(x2.data_ptr<float>(), dy.data_ptr(), norm_code(dy.scalar_type()), g.data_ptr<float>(),
+                                  mean.data_ptr<float>(), rstd.data_ptr<float>(), int(rows), int(n), dx.data_ptr<float>(),
+                                  dg.data_ptr<float>(), has_bias ? db.data_ptr<float>() : nullptr, 0, ws.data_ptr(), st));
+        return {dx, dg, db};
+    }
+};
+
+// The caller has checked that the kernels serve these tensors (layers/norm.py).
+Tensor layer_norm(const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias_, double eps) {
+    py::gil_scoped_release no_gil;
+    at::ScalarType out_t = at::kFloat;
+    if (at::autocast::is_autocast_enabled(at::kCUDA)) {
+        const at::ScalarType dt = at::autocast::get_autocast_dtype(at::kCUDA);
+        if (dt == at::kHalf || dt == at::kBFloat16) out_t = dt;
+    }
+    const Tensor bias = bias_ ? *bias_ : Tensor();
+    const at::Device dev = x.device();
+    c10::cuda::OptionalCUDAGuard guard(dev);
+    cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const int64_t n = x.size(-1), rows = x.numel() / n;
+    Tensor xc, y, mean, rstd;
+    {
+        at::NoGradGuard no_grad;
+        xc = x.contiguous();
+        y = at::detail::empty_cuda(x.sizes(), out_t, dev, std::nullopt);
+        mean = at::detail::empty_cuda({rows}, at::kFloat, dev, std::nullopt);
+        rstd = at::detail::empty_cuda({rows}, at::kFloat, dev, std::nullopt);
+        check_rc(sd_layernorm_fwd(xc.data_ptr<float>(), int(rows), int(n), weight.data_ptr<float>(),
+                                  bias.defined() ? bias.data_ptr<float>() : nullptr, float(eps), y.data_ptr(), norm_code(out_t),
+                                  mean.data_ptr<float>(), rstd.data_ptr<float>(), st));
+    }
+    if (!torch::autograd::compute_requires_grad(x, weight, bias)) return y;
+    std::shared_ptr<SparseDropLayerNormBackward> node(new SparseDropLayerNormBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, weight, bias));
+    node->x = SavedVariable(xc.is_same(x) ? x : xc, false);
+    node->weight = SavedVariable(weight, false);
+    node->mean = mean;
+    node->rstd = rstd;
+    node->has_bias = bias.defined();
+    node->shape = x.sizes().vec();
+    torch::autograd::set_history(y, node);
+    return y;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(sd_torch, m) {
+    m.doc() = "Native host path of the SparseDrop operator API";
+    py::register_exception_translator([](std::exception_ptr e) {
+        try {
+            if (e) std::rethrow_exception(e);
+        } catch (const SdError& err) {
+            static PyObject* type = py::module_::import("flash_dropout._lib").attr("SparseDropError").cast<py::object>().release().ptr();
+            PyErr_SetString(type, err.what());
+        }
+    });
+    register_node();
+    m.def("linear", &linear);
+    m.def("gemm", &gemm_dense);
+    m.def("gemm_dsd", &gemm_dsd);
+    m.def("gemm_sdd", &gemm_sdd);
+    m.def("layer_norm", &layer_norm);
+    m.def("status_word", [](int dev) { return status_tensor(dev); });
+    m.def("has_status_word", [](int dev) {
+        std::lock_guard<std::mutex> lock(state_mutex());
+        auto it = states().find(dev);
+        return it != states().end() && it->second.status.defined();
+    });
+    m.def("workspace", [](int dev, uint64_t stream) { return workspace_tensor(dev, reinterpret_cast<cudaStream_t>(stream)); });
+    m.def("workspaces", [](int dev) {
+        std::lock_guard<std::mutex> lock(state_mutex());
+        std::vector<Tensor> all;
+        for (auto& w : states()[dev].workspaces) all.push_back(w.second);
+        return all;
+    });
+}

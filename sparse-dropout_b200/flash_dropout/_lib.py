@@ -1,12 +1,13 @@
-"""ctypes binding of libsparsedrop.so (the C ABI declared in include/sparsedrop.h).
+"""ctypes binding of libsparsedrop.so (the C ABI declared in include/sparsedrop.h), and the torch extension on top of it.
 
-The library is built in-tree by ``csrc/build.sh`` into ``lib/libsparsedrop.so`` next to this
-package.  There is no fallback: if the library is missing, or no CUDA device is present when a
-kernel is requested, the call raises.
+Both are built in-tree by ``csrc/build.sh`` into ``lib/`` next to this package.  There is no fallback: if the library is missing, or no CUDA device is present when a
+kernel is requested, the call raises.  ``lib()`` is the C ABI itself; ``ext()`` is ``sd_torch.so`` (``csrc/sd_torch.cpp``), the
+native host path of the operators: what runs between a Python entry point and the C ABI on every call.
 """
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 from functools import lru_cache
 
@@ -14,6 +15,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(os.path.dirname(_HERE), "lib", "libsparsedrop.so")
+EXT_PATH = os.path.join(os.path.dirname(LIB_PATH), "sd_torch.so")
 
 SD_F16, SD_BF16, SD_F32 = 0, 1, 2
 SD_PLAN_ROWS, SD_PLAN_COLS = 0, 1
@@ -25,7 +27,7 @@ EXPORTS = (
     "sd_gemm_dsd_static_scratch", "sd_im2col_kept", "sd_col2im_kept", "sd_im2col_kept_panels", "sd_col2im_kept_panels",
     "sd_gemm_dsd_panels", "sd_gemm_sdd_kept_t_panels", "sd_selftest_bounded_wait", "sd_check_status",
     "sd_conv_fused_supported", "sd_conv_dsd_fwd", "sd_conv_dsd_dw",
-    "sd_gemm_dsd_relu", "sd_gemm_dsd_f32", "sd_gemm_sdd_relu_mask",
+    "sd_gemm_dsd_relu", "sd_gemm_dsd_f32", "sd_gemm_sdd_relu_mask", "sd_gemm_sdd_f32", "sd_cast16",
     "sd_plan_batch_desc_bytes", "sd_plan_batch_describe", "sd_plan_batch_launch", "sd_set_sm_margin",
     "sd_layernorm_fwd", "sd_layernorm_bwd_workspace_bytes", "sd_layernorm_bwd",
 )
@@ -98,6 +100,10 @@ def lib() -> C.CDLL:
     L.sd_gemm_dsd_f32.argtypes = mat * 3 + [i32, i32, i32, vp, i32, f32, i32, i32, vp, vp, vp]
     L.sd_gemm_sdd_relu_mask.restype = i32
     L.sd_gemm_sdd_relu_mask.argtypes = mat * 3 + [i32, i32, i32, vp, vp, i64, f32, i32, vp, vp, vp]
+    L.sd_gemm_sdd_f32.restype = i32
+    L.sd_gemm_sdd_f32.argtypes = L.sd_gemm_sdd_relu_mask.argtypes
+    L.sd_cast16.restype = i32
+    L.sd_cast16.argtypes = [vp, vp, i64, vp, vp, i64, i32, vp]
     L.sd_conv_fused_supported.restype = i32
     L.sd_conv_fused_supported.argtypes = [i32] * 12
     L.sd_conv_dsd_fwd.restype = i32
@@ -121,6 +127,23 @@ def lib() -> C.CDLL:
     L.sd_layernorm_bwd.restype = i32
     L.sd_layernorm_bwd.argtypes = [vp, vp, i32, vp, vp, vp, i32, i32, vp, vp, vp, i32, vp, vp]
     return L
+
+
+_ext = None
+
+
+def ext():
+    """The torch extension module (loads libsparsedrop.so with it)."""
+    global _ext
+    if _ext is None:
+        lib()
+        if not os.path.exists(EXT_PATH):
+            raise SparseDropError(f"{EXT_PATH} not found: build it with sparse-dropout_b200/csrc/build.sh")
+        spec = importlib.util.spec_from_file_location("sd_torch", EXT_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _ext = module
+    return _ext
 
 
 def check(rc: int) -> None:

@@ -253,26 +253,14 @@ class PlanBatch:
             self._ready = None
 
 
-_workspaces: dict = {}
-
-
 def workspace(device: torch.device) -> torch.Tensor:
     """Scratch for the split schedule of the GEMM kernel, one per (device, current stream).
 
     Launches that can overlap on the GPU must not share a workspace, hence the stream in the key.
     """
-    stream = _lib.stream_ptr(device)
-    key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
-    ws = _workspaces.get(key)
-    if ws is None:
-        with torch.cuda.device(device):
-            ws = torch.empty(_lib.lib().sd_workspace_bytes(), dtype=torch.uint8, device=device)
-            _lib.check(_lib.lib().sd_workspace_init(ws.data_ptr(), stream))
-        _workspaces[key] = ws
-    return ws
+    return _lib.ext().workspace(_dev_index(device), _lib.stream_ptr(device))
 
 
-_status_words: dict = {}
 SD_ERR_TIMEOUT = -4
 
 
@@ -283,12 +271,7 @@ def _dev_index(device: torch.device) -> int:
 def status_word(device: torch.device) -> torch.Tensor:
     """The device's failure-detection words (int32[4], word 0 is the status): every kernel launch of this module is
     given word 0, and a device-side wait that runs out of time records its code there instead of spinning on."""
-    idx = _dev_index(device)
-    w = _status_words.get(idx)
-    if w is None:
-        w = torch.zeros(4, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status_words[idx] = w
-    return w
+    return _lib.ext().status_word(_dev_index(device))
 
 
 def _status_ptr(device: torch.device) -> int:
@@ -308,9 +291,9 @@ def check_status(device: torch.device | int | None = None) -> None:
     elif isinstance(device, int):
         device = torch.device("cuda", device)
     idx = _dev_index(device)
-    w = _status_words.get(idx)
-    if w is None:
+    if not _lib.ext().has_status_word(idx):
         return                                  # nothing was ever launched on this device
+    w = _lib.ext().status_word(idx)
     L = _lib.lib()
     with _on_device(device):
         rc = L.sd_check_status(w.data_ptr(), _lib.stream_ptr(device))
@@ -318,9 +301,8 @@ def check_status(device: torch.device | int | None = None) -> None:
             return
         msg = L.sd_last_error().decode()
         if rc == SD_ERR_TIMEOUT:
-            for (d, stream), ws in _workspaces.items():
-                if d == idx:
-                    _lib.check(L.sd_workspace_init(ws.data_ptr(), _lib.stream_ptr(device)))
+            for ws in _lib.ext().workspaces(idx):
+                _lib.check(L.sd_workspace_init(ws.data_ptr(), _lib.stream_ptr(device)))
             w.zero_()
             torch.cuda.current_stream(device).synchronize()
     raise _lib.SparseDropError(f"libsparsedrop error {rc}: {msg}")
@@ -590,17 +572,12 @@ class GEMM:
             print(f"libsparsedrop {self.lib.sd_version()} loaded from {_lib.LIB_PATH}")
 
     def gemm(self, A: torch.Tensor, B: torch.Tensor) -> torch.Tensor:
-        return dense(A, B)
+        return _lib.ext().gemm(A, B)
 
     def gemm_dsd(self, A: torch.Tensor, B: torch.Tensor, mask: torch.Tensor, block_size: int,
                  scale: float) -> torch.Tensor:
-        _check_operand(A, "A")
-        plan = BlockPlan.from_mask(mask, A.size(0), A.size(1), block_size)
-        return dsd(A, B, plan, _lib.SD_PLAN_ROWS, scale)
+        return _lib.ext().gemm_dsd(A, B, mask, *_rep(block_size), scale)
 
     def gemm_sdd(self, A: torch.Tensor, B: torch.Tensor, mask: torch.Tensor, block_size: int,
                  scale: float) -> torch.Tensor:
-        _check_operand(A, "A")
-        _check_operand(B, "B")
-        plan = BlockPlan.from_mask(mask, A.size(0), B.size(0), block_size)
-        return sdd(A, B, plan, scale)
+        return _lib.ext().gemm_sdd(A, B, mask, *_rep(block_size), scale)

@@ -28,6 +28,7 @@ from flash_dropout import random as sd_random
 from flash_dropout.cuda.binding_gemm import (BlockPlan, _on_device, conv_dsd_dw, conv_dsd_fwd, conv_fused_supported,
                                              dsd_panels, sdd_kept_t_panels)
 
+from .blockwise_dropout_matmul_cuda import _autocast_input
 from .im2col_conv2d import conv_output_size
 
 
@@ -177,7 +178,7 @@ def blockwise_dropout_conv2d(input: torch.Tensor, kernel: torch.Tensor, block_si
     through the kept-block im2col stage."""
     if torch.is_autocast_enabled("cuda"):
         dt = torch.get_autocast_dtype("cuda")
-        input, kernel = input.to(dt), kernel.to(dt)
+        input, kernel = _autocast_input(input, dt), kernel.to(dt)
     with torch.autocast("cuda", enabled=False):
         return BlockwiseDropoutConv2dCUDA.apply(input, kernel, block_size, p, tuple(padding), tuple(stride),
                                                 tuple(dilation), plan, recompute_cols, fused)

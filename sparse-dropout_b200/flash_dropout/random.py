@@ -43,8 +43,8 @@ def set_state(state: dict) -> None:
     _state.update(state)
 
 
-def next_seed_offset() -> tuple[int, int]:
-    """(seed, offset) for the next mask; advances the counter."""
+def peek_seed_offset() -> tuple[int, int]:
+    """(seed, offset) for the next mask."""
     if _state["seed"] is None:
         ts = torch.initial_seed()
         if ts != _state["torch_seed"]:
@@ -53,9 +53,19 @@ def next_seed_offset() -> tuple[int, int]:
         seed = ts
     else:
         seed = _state["seed"]
-    off = _state["offset"]
-    _state["offset"] = off + 1
-    return seed & (2**64 - 1), (_state["subsequence"] << _SUBSEQ_SHIFT) + off
+    return seed & (2**64 - 1), (_state["subsequence"] << _SUBSEQ_SHIFT) + _state["offset"]
+
+
+def advance() -> None:
+    """Moves on to the following mask."""
+    _state["offset"] += 1
+
+
+def next_seed_offset() -> tuple[int, int]:
+    """(seed, offset) for the next mask; advances the counter."""
+    out = peek_seed_offset()
+    advance()
+    return out
 
 
 def enable_device_counter(device: torch.device, start: int = 0) -> torch.Tensor:
