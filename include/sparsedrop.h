@@ -277,6 +277,11 @@ int sd_col2im_kept_panels(const void* dcol_panels, int k_gemm, int N, int C, int
                           int pad_h, int pad_w, int stride_h, int stride_w, int dil_h, int dil_w,
                           void* dx, const void* plan, int dtype, void* stream);
 
+/* sd_col2im_kept_panels with dx in fp32: the gradient of an input kept in fp32 under autocast, without a cast kernel. */
+int sd_col2im_kept_panels_f32(const void* dcol_panels, int k_gemm, int N, int C, int H, int W, int R, int S,
+                              int pad_h, int pad_w, int stride_h, int stride_w, int dil_h, int dil_w,
+                              float* dx, const void* plan, int dtype, void* stream);
+
 /* DSD with the panel matrix P (pixels x kg) as A.  SD_PLAN_ROWS: C[pixels, N] = scale * (keep o col) . B^T with
  * B[N, kg] (the convolution's forward); SD_PLAN_COLS: C[kg, N] = scale * (keep o col)^T . B^T with B[N, pixels]
  * (its weight gradient). */
@@ -388,6 +393,30 @@ size_t sd_layernorm_bwd_workspace_bytes(int rows, int n);
 int sd_layernorm_bwd(const float* x, const void* dy, int dy_dtype, const float* gamma, const float* mean,
                      const float* rstd, int rows, int n, float* dx, float* dgamma, float* dbeta, int accumulate,
                      void* workspace, void* stream);
+
+/* ------------------------------------------------------------------------------------------
+ * AdamW over all parameters of a model in one launch (the reference trains with torch.optim.AdamW(fused=True),
+ * eval/llm/model.py:157-173).  Every tensor is contiguous fp32 in device memory, 16-byte aligned; `step` is its step counter
+ * (one float, as torch keeps it), which the launch advances by one.  Per element, with t the advanced counter:
+ *   p *= 1 - lr * weight_decay;  m += (g - m) * (1 - beta1);  v = beta2 * v + (1 - beta2) * g * g;
+ *   p -= lr / (1 - beta1^t) * m / (sqrt(v) / sqrt(1 - beta2^t) + eps)
+ * The table describes the tensors: fill a host buffer of sd_adamw_table_bytes() bytes with sd_adamw_table_fill(), copy it to
+ * device memory once (8-byte aligned), and pass the device copy to every step.  `hyper` is n_groups x 5 host doubles
+ * (lr, beta1, beta2, eps, weight_decay), read before the call returns.  n_chunks is the sum over the tensors of
+ * ceil(n / SD_ADAMW_CHUNK).  Steps on one table must not overlap.
+ * ------------------------------------------------------------------------------------------ */
+#define SD_ADAMW_MAX_GROUPS 8
+#define SD_ADAMW_CHUNK 2048
+typedef struct sd_adamw_entry {
+    float* p;
+    const float* g;
+    float *m, *v, *step;
+    int64_t n;
+    int32_t group, reserved;
+} sd_adamw_entry;
+size_t sd_adamw_table_bytes(const sd_adamw_entry* entries, int n);
+int sd_adamw_table_fill(void* host_table, const sd_adamw_entry* entries, int n);
+int sd_adamw_step(void* device_table, int64_t n_chunks, const double* hyper, int n_groups, void* stream);
 
 /*
  * Exercises the bounded device-side waits the kernels are built on, without a fault or a hang: a one-warp kernel

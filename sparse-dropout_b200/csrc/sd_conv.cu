@@ -11,6 +11,9 @@
 // built; nothing is taken from it.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <limits.h>
+
+#include <type_traits>
 
 #include "sd_common.h"
 #include "sd_plan.cuh"
@@ -203,13 +206,130 @@ __device__ __forceinline__ unsigned short from_float(float f, int is_bf16) {
     return is_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
 }
 
+// Eight consecutive results of dx starting at element 8 * i, as 16-bit values or in fp32 (an input kept in fp32 under
+// autocast takes its gradient in fp32).
+template <bool IS_BF16, bool OUT_F32>
+__device__ __forceinline__ void store_dx8(void* dx, long long i, const float (&acc)[8]) {
+    if (OUT_F32) {
+        float4* d = static_cast<float4*>(dx) + 2 * i;
+        d[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        d[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    } else {
+        uint32_t out[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (IS_BF16) {
+                __nv_bfloat162 v = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
+                out[j] = *reinterpret_cast<uint32_t*>(&v);
+            } else {
+                __half2 v = __floats2half2_rn(acc[2 * j], acc[2 * j + 1]);
+                out[j] = *reinterpret_cast<uint32_t*>(&v);
+            }
+        }
+        static_cast<uint4*>(dx)[i] = make_uint4(out[0], out[1], out[2], out[3]);
+    }
+}
+
+// col2im for any geometry, staged through shared memory.  A CTA owns a strip of SH input rows of CG channels of one image:
+// it copies the CG x R x S runs of dcolT that feed them (each run is contiguous along m, read as aligned 16-byte chunks;
+// chunks of dropped blocks become zeros) and then every thread gathers its results from there.  HBM-bound by design: each
+// kept entry is read once, in full sectors.  Reading the taps straight from memory instead, two bytes per lane with a
+// mask byte in front of every one, took 353 us on a 3x3 stride-2 layer (64 x 64 x 56 x 56) whose entries are 162 MB.
+struct StripGeom {
+    int SH, n_strips, CG, n_cgroups;
+    int pitch;              // elements per run in shared memory
+    int row_lanes;          // lanes that share one image row: a power of two, at most 32
+    int sh_h, sh_w;         // log2 of the strides, or -1
+};
+__device__ __forceinline__ int div_stride(int v, int stride, int sh, bool* exact) {
+    const int q = sh >= 0 ? v >> sh : v / stride;
+    *exact = q * stride == v;
+    return q;
+}
+template <bool IS_BF16, bool OUT_F32, int SMAX>
+__global__ void __launch_bounds__(kConvThreads) col2im_kept_strip_kernel(const unsigned short* __restrict__ dcolT,
+                                                                         void* __restrict__ dx, ConvGeom g, StripGeom sg,
+                                                                         const unsigned char* __restrict__ tile_mask) {
+    extern __shared__ __align__(16) unsigned short runs[];
+    const int RS = g.R * g.S, PQ = g.P * g.Q;
+    int u = blockIdx.x;
+    const int strip = u % sg.n_strips;
+    u /= sg.n_strips;
+    const int c0 = (u % sg.n_cgroups) * sg.CG, n = u / sg.n_cgroups;
+    const int cn = min(sg.CG, g.C - c0), h0 = strip * sg.SH, h1 = min(h0 + sg.SH, g.H);
+    // output rows that any tap of the strip's input rows reads
+    const int lo = h0 + g.pad_h - (g.R - 1) * g.dil_h, hi = h1 - 1 + g.pad_h;
+    const int p0 = max(lo <= 0 ? 0 : (lo + g.stride_h - 1) / g.stride_h, 0), p1 = min(hi / g.stride_h + 1, g.P);
+    const int m_first = n * PQ + p0 * g.Q, a0 = m_first & ~7;
+    const int nch = p1 > p0 ? (n * PQ + p1 * g.Q - a0 + 7) >> 3 : 0;
+    for (int e = threadIdx.x; e < cn * RS * nch; e += kConvThreads) {
+        const int row = e / nch, ch = e - row * nch;
+        const int k = c0 * RS + row, m = a0 + ch * 8;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (!(tile_mask && __ldg(tile_mask + (long long)(m >> 7) * g.Cb + (k >> 7))))
+            v = __ldg(reinterpret_cast<const uint4*>(dcolT + col_off(g, k, m)));
+        *reinterpret_cast<uint4*>(runs + row * sg.pitch + ch * 8) = v;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rows_per_warp = 32 / sg.row_lanes, sub = lane / sg.row_lanes, wl = lane - sub * sg.row_lanes;
+    const int base0 = n * PQ - a0;                                       // position of output pixel (0, 0) in a run
+    for (int w = wl; w < g.W; w += sg.row_lanes) {
+        int q[SMAX];                                                     // where tap s reads in its run, or INT_MIN
+#pragma unroll
+        for (int s = 0; s < SMAX; ++s) {
+            const int ww = w + g.pad_w - s * g.dil_w;
+            bool exact;
+            const int qq = div_stride(max(ww, 0), g.stride_w, sg.sh_w, &exact);
+            q[s] = (s < g.S && ww >= 0 && exact && qq < g.Q) ? qq + base0 : INT_MIN;
+        }
+        // (channel, input row) pairs of this thread, without a division per pair
+        const int rows = h1 - h0, step = (kConvThreads / 32) * rows_per_warp;
+        int first = warp * rows_per_warp + sub, cg = first / rows, h = first - cg * rows;
+        for (; cg < cn; h += step) {
+            while (h >= rows) { h -= rows; ++cg; }
+            if (cg >= cn) break;
+            const unsigned short* src = runs + cg * RS * sg.pitch;
+            const int top = h0 + h + g.pad_h;
+            float acc = 0.f;
+            if (g.dil_h == 1) {
+                // the filter rows that meet an output row: every stride_h-th one
+                int r = sg.sh_h == 0 ? 0 : sg.sh_h > 0 ? top & (g.stride_h - 1) : top % g.stride_h;
+                int p = sg.sh_h >= 0 ? (top - r) >> sg.sh_h : (top - r) / g.stride_h;
+                if (p >= g.P) { r += (p - g.P + 1) * g.stride_h; p = g.P - 1; }
+                for (; r < g.R && p >= 0; r += g.stride_h, --p) {
+                    const unsigned short* at = src + r * g.S * sg.pitch + p * g.Q;
+#pragma unroll
+                    for (int s = 0; s < SMAX; ++s)
+                        if (q[s] != INT_MIN) acc += to_float(at[s * sg.pitch + q[s]], IS_BF16);
+                }
+            } else {
+                for (int r = 0; r < g.R; ++r) {
+                    const int hh = top - r * g.dil_h;
+                    bool exact;
+                    const int p = div_stride(max(hh, 0), g.stride_h, sg.sh_h, &exact);
+                    if (hh < 0 || !exact || p >= g.P) continue;
+                    const unsigned short* at = src + r * g.S * sg.pitch + p * g.Q;
+#pragma unroll
+                    for (int s = 0; s < SMAX; ++s)
+                        if (q[s] != INT_MIN) acc += to_float(at[s * sg.pitch + q[s]], IS_BF16);
+                }
+            }
+            const long long i = ((long long)(n * g.C + c0 + cg) * g.H + h0 + h) * g.W + w;
+            if (OUT_F32) static_cast<float*>(dx)[i] = acc;
+            else static_cast<unsigned short*>(dx)[i] = from_float(acc, IS_BF16);
+        }
+    }
+}
+
 // Adjoint of the kept-block im2col: dx[n,c,h,w] = sum over the filter taps (r,s) that map (h,w) to an output
 // pixel (p,q) of dcolT[k(c,r,s)][m(n,p,q)], skipping dropped blocks (their entries are zero by definition).
-// One thread per input element, consecutive threads along w, so every tap is a coalesced read along m.
+// One thread per input element, consecutive threads along w.  Only for geometries whose strips do not fit shared memory
+// (see col2im_kept_strip_kernel).
 __global__ void __launch_bounds__(kConvThreads) col2im_kept_kernel(const unsigned short* __restrict__ dcolT,
-                                                                   unsigned short* __restrict__ dx, ConvGeom g,
+                                                                   void* __restrict__ dx, ConvGeom g,
                                                                    const unsigned char* __restrict__ tile_mask,
-                                                                   int is_bf16) {
+                                                                   int is_bf16, int out_f32) {
     const long long total = (long long)g.N * g.C * g.H * g.W;
     const int PQ = g.P * g.Q, RS = g.R * g.S;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -235,15 +355,16 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kept_kernel(const unsigne
                 acc += to_float(__ldg(dcolT + col_off(g, k, m)), is_bf16);
             }
         }
-        dx[i] = from_float(acc, is_bf16);
+        if (out_f32) static_cast<float*>(dx)[i] = acc;
+        else static_cast<unsigned short*>(dx)[i] = from_float(acc, is_bf16);
     }
 }
 
 // Fast col2im for unit strides with W % 8 == 0 and Q % 8 == 0: a thread owns 8 consecutive w of one (n, c, h);
 // every filter tap is one shifted 8-element window of one dcolT row, whose aligned chunks each lie in one block.
-template <bool IS_BF16>
+template <bool IS_BF16, bool OUT_F32>
 __global__ void __launch_bounds__(kConvThreads) col2im_kept_rows_kernel(const unsigned short* __restrict__ dcolT,
-                                                                        unsigned short* __restrict__ dx, ConvGeom g,
+                                                                        void* __restrict__ dx, ConvGeom g,
                                                                         const unsigned char* __restrict__ tile_mask) {
     const int WG = g.W >> 3;
     const unsigned total = unsigned(g.N) * g.C * g.H * WG;       // the host checks that this fits 32 bits
@@ -291,18 +412,7 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kept_rows_kernel(const un
                 }
             }
         }
-        uint32_t out[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (IS_BF16) {
-                __nv_bfloat162 v = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-                out[j] = *reinterpret_cast<uint32_t*>(&v);
-            } else {
-                __half2 v = __floats2half2_rn(acc[2 * j], acc[2 * j + 1]);
-                out[j] = *reinterpret_cast<uint32_t*>(&v);
-            }
-        }
-        *reinterpret_cast<uint4*>(dx + (long long)i * 8) = make_uint4(out[0], out[1], out[2], out[3]);
+        store_dx8<IS_BF16, OUT_F32>(dx, i, acc);
     }
 }
 
@@ -310,9 +420,9 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kept_rows_kernel(const un
 // owns 8 consecutive w of one (n, c, h) and reads, for each of the R x 3 taps, the aligned 8-pixel chunk of the tap's
 // dcolT row; taps s = 0 and s = 2 are that chunk shifted by one pixel, the pixel that falls off going to the
 // neighbour lane (which owns the neighbouring 8 pixels of the same image row).
-template <bool IS_BF16>
+template <bool IS_BF16, bool OUT_F32>
 __global__ void __launch_bounds__(kConvThreads) col2im_kept_s3_kernel(const unsigned short* __restrict__ dcolT,
-                                                                      unsigned short* __restrict__ dx, ConvGeom g,
+                                                                      void* __restrict__ dx, ConvGeom g,
                                                                       const unsigned char* __restrict__ tile_mask) {
     const int WG = g.W >> 3;                                     // lanes per image row; divides 32
     const unsigned total = unsigned(g.N) * g.C * g.H * WG;       // the host checks that this fits 32 bits
@@ -365,26 +475,15 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kept_s3_kernel(const unsi
             }
         }
         if (!live) continue;
-        uint32_t out[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (IS_BF16) {
-                __nv_bfloat162 v = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-                out[j] = *reinterpret_cast<uint32_t*>(&v);
-            } else {
-                __half2 v = __floats2half2_rn(acc[2 * j], acc[2 * j + 1]);
-                out[j] = *reinterpret_cast<uint32_t*>(&v);
-            }
-        }
-        *reinterpret_cast<uint4*>(dx + (long long)i * 8) = make_uint4(out[0], out[1], out[2], out[3]);
+        store_dx8<IS_BF16, OUT_F32>(dx, i, acc);
     }
 }
 
 // The same for 3 x 3 filters, unrolled over all nine taps: first the nine block-mask bytes, then the nine chunk loads
 // (independent of one another, so one memory round trip covers them all), then the arithmetic.
-template <bool IS_BF16>
+template <bool IS_BF16, bool OUT_F32>
 __global__ void __launch_bounds__(kConvThreads) col2im_kept_3x3_kernel(const unsigned short* __restrict__ dcolT,
-                                                                       unsigned short* __restrict__ dx, ConvGeom g,
+                                                                       void* __restrict__ dx, ConvGeom g,
                                                                        const unsigned char* __restrict__ tile_mask) {
     const int WG = g.W >> 3, wg_bits = 31 - __clz(WG);           // lanes per image row: a power of two up to 16
     const unsigned total = unsigned(g.N) * g.C * g.H * WG;       // the host checks that this fits 32 bits
@@ -453,18 +552,7 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kept_3x3_kernel(const uns
             }
         }
         if (!live) continue;
-        uint32_t out[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (IS_BF16) {
-                __nv_bfloat162 t = __floats2bfloat162_rn(acc[2 * j], acc[2 * j + 1]);
-                out[j] = *reinterpret_cast<uint32_t*>(&t);
-            } else {
-                __half2 t = __floats2half2_rn(acc[2 * j], acc[2 * j + 1]);
-                out[j] = *reinterpret_cast<uint32_t*>(&t);
-            }
-        }
-        *reinterpret_cast<uint4*>(dx + (long long)i * 8) = make_uint4(out[0], out[1], out[2], out[3]);
+        store_dx8<IS_BF16, OUT_F32>(dx, i, acc);
     }
 }
 
@@ -485,6 +573,38 @@ static int make_geom(ConvGeom* g, int N, int C, int H, int W, int R, int S, int 
     *g = ConvGeom{N, C, H, W, R, S, P, Q, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, int(M), int(K), ldm,
                   int((M + 127) / 128), (k_gemm + 127) / 128, panels ? 128 : ldm, panels ? (long long)k_gemm * 128 : 0};
     return SD_OK;
+}
+
+// Strip height and channels per CTA of the staged col2im, and its shared memory; false if the geometry does not fit.
+// Strips are as tall as 40 KB of runs allow (the overlap of neighbouring strips is read twice); small images take several
+// channels per CTA, so that a CTA has at least about a thousand results to gather.
+static bool strip_geom(const ConvGeom& g, uintptr_t src, StripGeom* sg, int* bytes) {
+    if (g.S > 7 || (src & 15)) return false;
+    const int RS = g.R * g.S;
+    auto run_elems = [&](int SH) {
+        long long np = (SH - 1 + (long long)(g.R - 1) * g.dil_h) / g.stride_h + 2;
+        if (np > g.P) np = g.P;
+        return ((np * g.Q + 14) & ~7ll) + 8;                  // start and end rounded to chunks of 8
+    };
+    int SH = g.H;
+    while (SH > 1 && run_elems(SH) * RS * 2 > 40 * 1024) SH = (SH + 1) / 2;
+    const long long one = run_elems(SH) * RS * 2;
+    if (one > 44 * 1024) return false;
+    int CG = 1;
+    while (CG * 2 <= g.C && one * CG * 2 <= 24 * 1024 && (long long)CG * SH * g.W < 1024) CG *= 2;
+    sg->SH = SH;
+    sg->n_strips = (g.H + SH - 1) / SH;
+    sg->CG = CG;
+    sg->n_cgroups = (g.C + CG - 1) / CG;
+    sg->pitch = int(run_elems(SH));
+    sg->row_lanes = 1;
+    while (sg->row_lanes < g.W && sg->row_lanes < 32) sg->row_lanes *= 2;
+    auto log2_or = [](int v) { int l = 0; while ((1 << l) < v) ++l; return (1 << l) == v ? l : -1; };
+    sg->sh_h = log2_or(g.stride_h);
+    sg->sh_w = log2_or(g.stride_w);
+    if ((long long)g.N * sg->n_cgroups * sg->n_strips > (1ll << 31) - 1) return false;
+    *bytes = int(one * CG);
+    return true;
 }
 
 }  // namespace sd
@@ -526,7 +646,7 @@ static int im2col_kept_impl(const void* x, int N, int C, int H, int W, int R, in
 
 static int col2im_kept_impl(const void* dcolT, int64_t ldm, int k_gemm, int N, int C, int H, int W, int R, int S, int pad_h,
                             int pad_w, int stride_h, int stride_w, int dil_h, int dil_w, void* dx, const void* plan,
-                            int dtype, void* stream, bool panels) {
+                            int dtype, void* stream, bool panels, bool out_f32 = false) {
     if (!dcolT || !dx) return sd::fail(SD_ERR_INVALID_ARG, "dcolT or dx is null");
     if (dtype != SD_F16 && dtype != SD_BF16) return sd::fail(SD_ERR_INVALID_ARG, "dtype must be SD_F16 or SD_BF16");
     sd::ConvGeom g;
@@ -544,27 +664,31 @@ static int col2im_kept_impl(const void* dcolT, int64_t ldm, int k_gemm, int N, i
     long long blocks = (total + sd::kConvThreads - 1) / sd::kConvThreads;
     int grid = int(blocks < (long long)sms * 16 ? blocks : (long long)sms * 16);
     const bool s3_path = rows_path && S == 3 && dil_w == 1 && pad_w == 1 && W <= 128 && 128 % W == 0;
-    if (s3_path && R == 3 && dtype == SD_BF16)
-        sd::col2im_kept_3x3_kernel<true><<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const unsigned short*>(dcolT), static_cast<unsigned short*>(dx), g, mask);
-    else if (s3_path && R == 3)
-        sd::col2im_kept_3x3_kernel<false><<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const unsigned short*>(dcolT), static_cast<unsigned short*>(dx), g, mask);
-    else if (s3_path && dtype == SD_BF16)
-        sd::col2im_kept_s3_kernel<true><<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const unsigned short*>(dcolT), static_cast<unsigned short*>(dx), g, mask);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const unsigned short* src = static_cast<const unsigned short*>(dcolT);
+    auto by_type = [&](auto&& launch) {                      // launch(bf16, fp32 result) as compile-time flags
+        if (dtype == SD_BF16) {
+            if (out_f32) launch(std::true_type{}, std::true_type{}); else launch(std::true_type{}, std::false_type{});
+        } else {
+            if (out_f32) launch(std::false_type{}, std::true_type{}); else launch(std::false_type{}, std::false_type{});
+        }
+    };
+    sd::StripGeom sg;
+    int strip_bytes = 0;
+    if (s3_path && R == 3)
+        by_type([&](auto bf, auto f32) { sd::col2im_kept_3x3_kernel<bf.value, f32.value><<<grid, sd::kConvThreads, 0, st>>>(src, dx, g, mask); });
     else if (s3_path)
-        sd::col2im_kept_s3_kernel<false><<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const unsigned short*>(dcolT), static_cast<unsigned short*>(dx), g, mask);
-    else if (rows_path && dtype == SD_BF16)
-        sd::col2im_kept_rows_kernel<true><<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const unsigned short*>(dcolT), static_cast<unsigned short*>(dx), g, mask);
+        by_type([&](auto bf, auto f32) { sd::col2im_kept_s3_kernel<bf.value, f32.value><<<grid, sd::kConvThreads, 0, st>>>(src, dx, g, mask); });
     else if (rows_path)
-        sd::col2im_kept_rows_kernel<false><<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const unsigned short*>(dcolT), static_cast<unsigned short*>(dx), g, mask);
-    else
-        sd::col2im_kept_kernel<<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const unsigned short*>(dcolT), static_cast<unsigned short*>(dx), g, mask, dtype == SD_BF16);
+        by_type([&](auto bf, auto f32) { sd::col2im_kept_rows_kernel<bf.value, f32.value><<<grid, sd::kConvThreads, 0, st>>>(src, dx, g, mask); });
+    else if (sd::strip_geom(g, reinterpret_cast<uintptr_t>(dcolT), &sg, &strip_bytes)) {
+        const unsigned n_cta = unsigned(N) * sg.n_cgroups * sg.n_strips;
+        by_type([&](auto bf, auto f32) {
+            if (S <= 3) sd::col2im_kept_strip_kernel<bf.value, f32.value, 3><<<n_cta, sd::kConvThreads, strip_bytes, st>>>(src, dx, g, sg, mask);
+            else sd::col2im_kept_strip_kernel<bf.value, f32.value, 7><<<n_cta, sd::kConvThreads, strip_bytes, st>>>(src, dx, g, sg, mask);
+        });
+    } else
+        sd::col2im_kept_kernel<<<grid, sd::kConvThreads, 0, st>>>(src, dx, g, mask, dtype == SD_BF16, out_f32);
     SD_CUDA_TRY(cudaGetLastError());
     return SD_OK;
 }
@@ -590,6 +714,13 @@ int sd_col2im_kept(const void* dcolT, int64_t ldm, int k_gemm, int N, int C, int
                    void* stream) {
     return col2im_kept_impl(dcolT, ldm, k_gemm, N, C, H, W, R, S, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, dx,
                             plan, dtype, stream, false);
+}
+
+int sd_col2im_kept_panels_f32(const void* dcol_panels, int k_gemm, int N, int C, int H, int W, int R, int S, int pad_h,
+                              int pad_w, int stride_h, int stride_w, int dil_h, int dil_w, float* dx, const void* plan,
+                              int dtype, void* stream) {
+    return col2im_kept_impl(dcol_panels, 0, k_gemm, N, C, H, W, R, S, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w,
+                            dx, plan, dtype, stream, true, true);
 }
 
 int sd_col2im_kept_panels(const void* dcol_panels, int k_gemm, int N, int C, int H, int W, int R, int S, int pad_h,

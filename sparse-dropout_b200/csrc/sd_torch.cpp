@@ -1,5 +1,6 @@
 // The operator API's path from torch tensors to libsparsedrop.so, in native code: argument checks, the casts under
-// autocast, the mask draw, the launches and the autograd nodes of a SparseDrop linear and of the LayerNorm in front of it.
+// autocast, the mask draw, the launches and the autograd nodes of a SparseDrop linear, of the convolution
+// and of the LayerNorm in front of them.
 //
 // A small layer is bound by the host: its four kernels take 31 us at 512^3 while the same sequence issued from Python
 // (ctypes calls, a Python autograd.Function, tensor bookkeeping) took 197 us per forward + backward.  Everything between
@@ -20,6 +21,9 @@
 #include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <pybind11/stl.h>
+
+#include <array>
 #include <mutex>
 #include <optional>
 #include <unordered_map>
@@ -167,7 +171,8 @@ struct CastEntry {
     c10::weak_intrusive_ptr<c10::TensorImpl> owner, copy;
     uint32_t version;
     at::ScalarType dt;
-    int64_t offset, size[2], stride[2];
+    int64_t offset;
+    std::vector<int64_t> size, stride;
     cudaStream_t stream;
 };
 struct CastCache {
@@ -175,8 +180,7 @@ struct CastCache {
     static Tensor owner_of(const Tensor& x) { return x.is_view() ? Tensor(x._base()) : x; }
     Tensor find(const Tensor& x, at::ScalarType dt, cudaStream_t stream) {
         if (!e || x.is_inference() || e->dt != dt || e->stream != stream || e->version != x._version() || e->offset != x.storage_offset()) return {};
-        for (int i = 0; i < 2; ++i)
-            if (e->size[i] != x.size(i) || e->stride[i] != x.stride(i)) return {};
+        if (x.sizes() != at::IntArrayRef(e->size) || x.strides() != at::IntArrayRef(e->stride)) return {};
         auto own = e->owner.lock();
         if (!own || own.get() != owner_of(x).unsafeGetTensorImpl()) return {};
         auto copy = e->copy.lock();
@@ -186,7 +190,7 @@ struct CastCache {
         if (x.is_inference()) return;
         e.emplace(CastEntry{c10::weak_intrusive_ptr<c10::TensorImpl>(owner_of(x).getIntrusivePtr()),
                             c10::weak_intrusive_ptr<c10::TensorImpl>(x16.getIntrusivePtr()), uint32_t(x._version()), x16.scalar_type(),
-                            x.storage_offset(), {x.size(0), x.size(1)}, {x.stride(0), x.stride(1)}, stream});
+                            x.storage_offset(), x.sizes().vec(), x.strides().vec(), stream});
     }
 };
 
@@ -223,6 +227,7 @@ struct SparseDropLinearBackward : public Node {
     int64_t block_m = 0, block_k = 0;
     bool pair_block = false;
     int64_t M = 0, K = 0, N = 0;
+    std::vector<int64_t> lead;                     // shape of an input that is not 2-D
     double p = 0;
     bool x_f32 = false, w_f32 = false;             // the layer's own tensors are fp32: their gradients leave in fp32
     Options opt;
@@ -238,22 +243,25 @@ struct SparseDropLinearBackward : public Node {
 
 variable_list SparseDropLinearBackward::apply(variable_list&& grads) {
     at::NoGradGuard no_grad;
-    const Tensor x16 = x.unpack(), w16 = w.unpack();
+    Tensor x16 = x.unpack();
+    const Tensor w16 = w.unpack();
+    if (x16.dim() != 2) x16 = x16.view({M, K});
     const at::Device dev = x16.device();
     c10::cuda::OptionalCUDAGuard guard(dev);
     const Launch L(dev);
     const float scale = float(1.0 / (1.0 - p));
     const int dt = dtype_code(x16.scalar_type());
     const Tensor pl = plan.defined() ? plan : draw_plan(draw, M, K, dev, L.stream);
-    Tensor dy = grads[0].defined() ? grads[0] : at::zeros({M, N}, x16.options());
+    Tensor dy = grads[0].defined() ? grads[0] : at::zeros({M, N}, x16.options());     // (any rank: only the element count matters)
     if (dy.scalar_type() != x16.scalar_type()) dy = dy.to(x16.scalar_type());
     if (opt.relu && !opt.premasked) dy = at::threshold_backward(dy, y.unpack(shared_from_this()), 0);
-    dy = operand(dy);
+    dy = operand(dy.dim() == 2 ? dy : dy.reshape({M, N}));
     const Mat mdy = mat(dy), mx = mat(x16), mdyt = mat_t(dy), mxt = mat_t(x16), mwt = mat_t(w16);
     Tensor dx, dw;
     if (task_should_compute_output(0)) {
         // dx (M, K) = keep o (dy (M, N) . W (N, K)) * scale
-        dx = empty2(M, K, x_f32 ? at::kFloat : x16.scalar_type(), dev);
+        const at::ScalarType t = x_f32 ? at::kFloat : x16.scalar_type();
+        dx = lead.empty() ? empty2(M, K, t, dev) : Tensor(at::detail::empty_cuda(lead, t, dev, std::nullopt));
         void* mask = opt.input_relu ? mx.p : nullptr;
         if (x_f32)
             check_rc(sd_gemm_sdd_f32(mdy.p, mdy.rs, mdy.cs, mwt.p, mwt.rs, mwt.cs, dx.data_ptr<float>(), K, 1, int(M), int(K), int(N),
@@ -290,7 +298,7 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
               int64_t rep_r, int64_t rep_c, bool pair_block, double p, uint64_t seed, uint64_t offset,
               const std::optional<Tensor>& counter, bool relu, bool input_relu, bool premasked,
               const std::optional<Tensor>& wgrad, bool wgrad_acc, py::handle notify, bool recompute,
-              const std::optional<Tensor>& weight_lowp) {
+              const std::optional<Tensor>& weight_lowp, bool any_rank) {
     Options opt;
     opt.relu = relu;
     opt.input_relu = input_relu;
@@ -302,7 +310,7 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     }
     py::gil_scoped_release no_gil;
     if (!input_.is_cuda() || !weight_.is_cuda()) bad("input and weight must be CUDA");   // no CPU path, as gemm_binding.cu:19
-    if (input_.dim() != 2 || weight_.dim() != 2) bad("input and weight must be 2D");
+    if ((any_rank ? input_.dim() < 1 : input_.dim() != 2) || weight_.dim() != 2) bad("input and weight must be 2D");
     if (input_.device() != weight_.device()) bad("A and B must be on the same device");
     const at::Device dev = input_.device();
     c10::cuda::OptionalCUDAGuard guard(dev);
@@ -332,7 +340,7 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
         bad(std::string("input (") + c10::toString(x16.scalar_type()) + ") and weight (" + c10::toString(w16.scalar_type()) +
             ") must have the same dtype");
     const int dt = dtype_code(x16.scalar_type());
-    const int64_t M = x16.size(0), K = x16.size(1), N = w16.size(0);
+    const int64_t K = x16.size(-1), M = K ? x16.numel() / K : 0, N = w16.size(0);
     if (K % 8 || N % 8) bad("in_features and out_features must be multiples of 8 (16-byte TMA rows)");
     if (w16.size(1) != K)
         bad("reduction dimensions differ: A is (" + std::to_string(M) + ", " + std::to_string(K) + "), B is (" + std::to_string(N) +
@@ -348,7 +356,8 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     Draw d;
     {
         at::NoGradGuard no_grad;
-        xs = operand(x16);
+        // leading dimensions are rows: no view goes through autograd for them
+        xs = operand(x16.dim() == 2 ? x16 : x16.reshape({M, K}));
         ws = operand(w16);
         if (input_relu && xs.stride(1) != 1) xs = xs.contiguous();
         if (plan_ && plan_->defined()) {
@@ -364,7 +373,13 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
         d.rep_c = int(rep_c);
         d.p = float(p);
         if (!plan.defined()) plan = draw_plan(d, M, K, dev, L.stream);
-        out = empty2(M, N, xs.scalar_type(), dev);
+        if (input.dim() == 2)
+            out = empty2(M, N, xs.scalar_type(), dev);
+        else {
+            std::vector<int64_t> shape = input.sizes().vec();
+            shape.back() = N;
+            out = at::detail::empty_cuda(shape, xs.scalar_type(), dev, std::nullopt);
+        }
         const Mat a = mat(xs), b = mat(ws);
         check_rc((relu ? sd_gemm_dsd_relu : sd_gemm_dsd)(a.p, a.rs, a.cs, b.p, b.rs, b.cs, out.data_ptr(), N, 1, int(M), int(N), int(K),
                                                          plan.data_ptr(), SD_PLAN_ROWS, float(1.0 / (1.0 - p)), dt, L.ws, L.status,
@@ -373,7 +388,9 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     if (!needs_grad) return out;
     std::shared_ptr<SparseDropLinearBackward> node(new SparseDropLinearBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(input, weight));
-    node->x = SavedVariable(xs.is_same(x16) && x16.is_same(input) ? input : xs, false);
+    // an input that went to the kernel as it is (possibly as a 2-D view of itself) is saved as the variable it is
+    const bool own = x16.is_same(input) && xs.data_ptr() == input.data_ptr() && (input.dim() == 2 ? xs.is_same(x16) : input.is_contiguous());
+    node->x = SavedVariable(own ? input : xs, false);
     node->w = SavedVariable(ws.is_same(w16) && w16.is_same(weight) ? weight : ws, false);
     node->draw = d;
     node->block_m = rep_r * TILE;
@@ -384,6 +401,7 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     node->K = K;
     node->N = N;
     node->p = p;
+    if (input.dim() != 2) node->lead = input.sizes().vec();
     node->x_f32 = input.scalar_type() == at::kFloat;
     node->w_f32 = weight.scalar_type() == at::kFloat;
     node->opt = std::move(opt);
@@ -491,6 +509,181 @@ Tensor gemm_sdd(const Tensor& A, const Tensor& B, const Tensor& mask, int64_t re
     return C;
 }
 
+// ---------------------------------------------------------------- a SparseDrop convolution
+// Blockwise dropout on the im2col matrix (M = N*P*Q rows, K = C*R*S columns in unfold order); see
+// functional/blockwise_dropout_conv2d.py for the stages and the semantics.
+struct ConvGeometry {
+    int N, C, H, W, R, S, ph, pw, sh, sw, dh, dw, P, Q, Ko;
+    int M, K, Kg, Kog;                             // Kg, Kog: K and Ko rounded up to what the kernels take
+};
+#define SD_CONV_GEOM(g) g.N, g.C, g.H, g.W, g.R, g.S, g.ph, g.pw, g.sh, g.sw, g.dh, g.dw
+
+Tensor im2col_panels(const Tensor& x, const ConvGeometry& g, const Tensor& plan, cudaStream_t stream) {
+    Tensor col = at::detail::empty_cuda({tiles_of(g.M), g.Kg, TILE}, x.scalar_type(), x.device(), std::nullopt);
+    if (g.Kg > g.K) col.slice(1, g.K).zero_();
+    check_rc(sd_im2col_kept_panels(x.data_ptr(), SD_CONV_GEOM(g), col.data_ptr(), g.Kg, plan.data_ptr(), stream));
+    return col;
+}
+
+struct SparseDropConv2dBackward : public Node {
+    SavedVariable x, w2d, cols;
+    Tensor plan;
+    ConvGeometry g;
+    double p = 0;
+    bool fused = false, has_cols = false, x_f32 = false, w_f32 = false;
+
+    std::string name() const override { return "SparseDropConv2dBackward"; }
+    void release_variables() override {
+        x.reset_data();
+        w2d.reset_data();
+        cols.reset_data();
+    }
+    variable_list apply(variable_list&& grads) override {
+        at::NoGradGuard no_grad;
+        const Tensor x16 = x.unpack(), w = w2d.unpack();
+        const at::Device dev = x16.device();
+        c10::cuda::OptionalCUDAGuard guard(dev);
+        const Launch L(dev);
+        const at::ScalarType t = x16.scalar_type();
+        const int dt = dtype_code(t);
+        const float scale = float(1.0 / (1.0 - p));
+        Tensor dy = grads[0].defined() ? grads[0] : at::zeros({g.N, g.Ko, g.P, g.Q}, x16.options());
+        if (dy.scalar_type() != t) dy = dy.to(t);
+        dy = dy.permute({0, 2, 3, 1}).reshape({g.M, g.Ko});          // free for channels-last gradients
+        if (g.Kog != g.Ko) dy = at::constant_pad_nd(dy, {0, g.Kog - g.Ko});
+        dy = dy.contiguous();
+        if (reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16) dy = dy.clone();
+        const Mat mdy = mat(dy);
+        Tensor dx, dwt;
+        if (task_should_compute_output(1)) {
+            Tensor dw = empty2(g.Kog, g.Kg, t, dev);
+            if (fused)
+                check_rc(sd_conv_dsd_dw(x16.data_ptr(), SD_CONV_GEOM(g), mdy.p, mdy.rs, mdy.cs, dw.data_ptr(), g.Kg, 1, g.Kog,
+                                        plan.data_ptr(), scale, dt, L.ws, L.status, L.stream));
+            else {
+                const Tensor col = has_cols ? cols.unpack() : im2col_panels(x16, g, plan, L.stream);
+                check_rc(sd_gemm_dsd_panels(col.data_ptr(), g.M, g.Kg, mdy.p, mdy.cs, mdy.rs, dw.data_ptr(), 1, g.Kg, g.Kog,
+                                            plan.data_ptr(), SD_PLAN_COLS, scale, dt, L.ws, L.status, L.stream));
+            }
+            if (g.Kog != g.Ko || g.Kg != g.K) dw = dw.slice(0, 0, g.Ko).slice(1, 0, g.K);
+            if (w_f32) dw = dw.to(at::kFloat);
+            dwt = dw.reshape({g.Ko, g.C, g.R, g.S});
+        }
+        if (task_should_compute_output(0)) {
+            // kept blocks of dcolP = W2d^T . dY^T, then the adjoint gather
+            Tensor dcol = at::detail::empty_cuda({tiles_of(g.M), g.Kg, TILE}, t, dev, std::nullopt);
+            const Mat mwt = mat_t(w);
+            check_rc(sd_gemm_sdd_kept_t_panels(mwt.p, mwt.rs, mwt.cs, mdy.p, mdy.rs, mdy.cs, dcol.data_ptr(), g.Kg, g.M, g.Kog,
+                                               plan.data_ptr(), scale, dt, L.ws, L.status, L.stream));
+            dx = at::detail::empty_cuda({g.N, g.C, g.H, g.W}, x_f32 ? at::kFloat : t, dev, std::nullopt);
+            if (x_f32)
+                check_rc(sd_col2im_kept_panels_f32(dcol.data_ptr(), g.Kg, SD_CONV_GEOM(g), dx.data_ptr<float>(), plan.data_ptr(), dt, L.stream));
+            else
+                check_rc(sd_col2im_kept_panels(dcol.data_ptr(), g.Kg, SD_CONV_GEOM(g), dx.data_ptr(), plan.data_ptr(), dt, L.stream));
+        }
+        return {dx, dwt};
+    }
+};
+
+Tensor conv2d(const Tensor& input_, const Tensor& kernel_, const std::optional<Tensor>& plan_, int64_t plan_R, int64_t plan_C,
+              int64_t rep_r, int64_t rep_c, double p, uint64_t seed, uint64_t offset, const std::optional<Tensor>& counter,
+              std::array<int64_t, 2> padding, std::array<int64_t, 2> stride, std::array<int64_t, 2> dilation, bool recompute_cols,
+              bool want_fused) {
+    py::gil_scoped_release no_gil;
+    if (!input_.is_cuda() || !kernel_.is_cuda()) bad("input and kernel must be CUDA");
+    const Tensor &input = input_, &kernel = kernel_;
+    const bool amp = at::autocast::is_autocast_enabled(at::kCUDA);
+    const at::ScalarType t = amp ? at::autocast::get_autocast_dtype(at::kCUDA) : input.scalar_type();
+    if (!amp && input.scalar_type() != kernel.scalar_type())
+        bad(std::string("input (") + c10::toString(input.scalar_type()) + ") and kernel (" + c10::toString(kernel.scalar_type()) +
+            ") must have the same dtype");
+    const int dt = dtype_code(t);
+    if (input.dim() != 4 || kernel.dim() != 4) bad("input must be NCHW and kernel [out, in, R, S]");
+    ConvGeometry g;
+    g.N = int(input.size(0)); g.C = int(input.size(1)); g.H = int(input.size(2)); g.W = int(input.size(3));
+    g.Ko = int(kernel.size(0)); g.R = int(kernel.size(2)); g.S = int(kernel.size(3));
+    if (kernel.size(1) != g.C) bad("kernel expects " + std::to_string(kernel.size(1)) + " input channels, input has " + std::to_string(g.C));
+    g.ph = int(padding[0]); g.pw = int(padding[1]); g.sh = int(stride[0]); g.sw = int(stride[1]); g.dh = int(dilation[0]); g.dw = int(dilation[1]);
+    if (g.sh <= 0 || g.sw <= 0) bad("stride must be positive");
+    g.P = (g.H + 2 * g.ph - g.dh * (g.R - 1) - 1) / g.sh + 1;
+    g.Q = (g.W + 2 * g.pw - g.dw * (g.S - 1) - 1) / g.sw + 1;
+    const int64_t M = int64_t(g.N) * g.P * g.Q, K = int64_t(g.C) * g.R * g.S;
+    if (g.P <= 0 || g.Q <= 0 || M > (1ll << 30) || K > (1ll << 30)) bad("the filter does not fit the padded input, or the im2col matrix is too large");
+    g.M = int(M);
+    g.K = int(K);
+    g.Kg = (g.K + 63) & ~63;                        // the im2col matrix is kept in panels: k extent a multiple of 64
+    g.Kog = (g.Ko + 7) & ~7;
+    const at::Device dev = input.device();
+    c10::cuda::OptionalCUDAGuard guard(dev);
+    const Launch L(dev);
+    Tensor plan, x16, w2d, y2d, cols;
+    bool fused;
+    {
+        at::NoGradGuard no_grad;
+        if (plan_ && plan_->defined()) {
+            if (plan_R != tiles_of(g.M) || plan_C != tiles_of(g.Kg))
+                bad("plan grid (" + std::to_string(plan_R) + ", " + std::to_string(plan_C) + ") does not match the " + std::to_string(g.M) +
+                    " x " + std::to_string(g.Kg) + " im2col matrix");
+            plan = *plan_;
+        } else {
+            Draw d;
+            d.seed = seed;
+            d.offset = offset;
+            d.counter = counter && counter->defined() ? static_cast<uint64_t*>(counter->data_ptr()) : nullptr;
+            d.rep_r = int(rep_r);
+            d.rep_c = int(rep_c);
+            d.p = float(p);
+            plan = draw_plan(d, g.M, g.Kg, dev, L.stream);
+        }
+        // 16-byte rows for TMA; zero padding changes nothing
+        const bool pad_w2d = g.Kg != g.K || g.Kog != g.Ko, cast_x = input.scalar_type() != t, cast_w = kernel.scalar_type() != t;
+        x16 = input;
+        Tensor kflat = kernel.reshape({g.Ko, g.K}), k16 = kflat;
+        if (cast_x || (cast_w && !pad_w2d)) cast_pair(cast_x ? input : Tensor(), x16, cast_w && !pad_w2d ? kflat : Tensor(), k16, t, L.stream);
+        if (pad_w2d) {
+            w2d = at::zeros({g.Kog, g.Kg}, kernel.options().dtype(t));
+            w2d.slice(0, 0, g.Ko).slice(1, 0, g.K).copy_(kflat);
+        } else
+            w2d = k16.contiguous();
+        x16 = x16.contiguous();
+        if (reinterpret_cast<uintptr_t>(x16.data_ptr()) % 16) x16 = x16.clone();
+        if (reinterpret_cast<uintptr_t>(w2d.data_ptr()) % 16) w2d = w2d.clone();
+        y2d = empty2(g.M, g.Kog, t, dev);
+        const Mat mw = mat(w2d);
+        const float scale = float(1.0 / (1.0 - p));
+        fused = want_fused && sd_conv_fused_supported(SD_CONV_GEOM(g));
+        if (fused)
+            check_rc(sd_conv_dsd_fwd(x16.data_ptr(), SD_CONV_GEOM(g), mw.p, mw.rs, mw.cs, y2d.data_ptr(), g.Kog, 1, g.Kog, plan.data_ptr(),
+                                     scale, dt, L.ws, L.status, L.stream));
+        else {
+            cols = im2col_panels(x16, g, plan, L.stream);
+            check_rc(sd_gemm_dsd_panels(cols.data_ptr(), g.M, g.Kg, mw.p, mw.rs, mw.cs, y2d.data_ptr(), g.Kog, 1, g.Kog, plan.data_ptr(),
+                                        SD_PLAN_ROWS, scale, dt, L.ws, L.status, L.stream));
+        }
+    }
+    // an NCHW-shaped view of y2d with channels-last strides
+    Tensor out;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        out = y2d.as_strided({g.N, g.Ko, g.P, g.Q}, {int64_t(g.P) * g.Q * g.Kog, 1, int64_t(g.Q) * g.Kog, g.Kog});
+    }
+    if (!torch::autograd::compute_requires_grad(input, kernel)) return out;
+    std::shared_ptr<SparseDropConv2dBackward> node(new SparseDropConv2dBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(input, kernel));
+    node->x = SavedVariable(x16.is_same(input) ? input : x16, false);
+    node->w2d = SavedVariable(w2d, false);
+    node->has_cols = !fused && !recompute_cols;
+    if (node->has_cols) node->cols = SavedVariable(cols, false);
+    node->plan = plan;
+    node->g = g;
+    node->p = p;
+    node->fused = fused;
+    node->x_f32 = input.scalar_type() == at::kFloat;
+    node->w_f32 = kernel.scalar_type() == at::kFloat;
+    torch::autograd::set_history(out, node);
+    return out;
+}
+
 // ---------------------------------------------------------------- LayerNorm
 int norm_code(at::ScalarType t) { return t == at::kHalf ? SD_F16 : t == at::kBFloat16 ? SD_BF16 : SD_F32; }
 
@@ -529,9 +722,18 @@ struct SparseDropLayerNormBackward : public Node {
     }
 };
 
-// The caller has checked that the kernels serve these tensors (layers/norm.py).
-Tensor layer_norm(const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias_, double eps) {
+// Nothing if the kernels do not serve these tensors: fp32 rows of up to 1024 elements, a multiple of 4, on a CUDA device.
+std::optional<Tensor> layer_norm(const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias_, double eps) {
     py::gil_scoped_release no_gil;
+    {
+        const int64_t w = x.dim() ? x.size(-1) : 0;
+        const auto plain = [&](const Tensor& t) {
+            return t.scalar_type() == at::kFloat && t.is_contiguous() && t.dim() == 1 && t.size(0) == w && t.device() == x.device();
+        };
+        if (!x.is_cuda() || x.scalar_type() != at::kFloat || w % 4 || w <= 0 || w > 1024 || x.numel() == 0 || x.numel() / w >= (1ll << 31) ||
+            !plain(weight) || (bias_ && !plain(*bias_)))
+            return std::nullopt;
+    }
     at::ScalarType out_t = at::kFloat;
     if (at::autocast::is_autocast_enabled(at::kCUDA)) {
         const at::ScalarType dt = at::autocast::get_autocast_dtype(at::kCUDA);
@@ -566,6 +768,51 @@ Tensor layer_norm(const Tensor& x, const Tensor& weight, const std::optional<Ten
     return y;
 }
 
+// ---------------------------------------------------------------- AdamW
+// The tensors of one optimizer, described to the kernel once; a step checks that none of them has moved since.
+struct AdamW {
+    std::vector<std::array<Tensor, 5>> tensors;    // p, g, m, v, step
+    std::vector<std::array<void*, 5>> where;
+    Tensor table;
+    int64_t chunks = 0;
+
+    AdamW(const std::vector<std::array<Tensor, 5>>& t, const std::vector<int64_t>& groups) : tensors(t) {
+        std::vector<sd_adamw_entry> e;
+        for (size_t i = 0; i < t.size(); ++i) {
+            std::array<void*, 5> at;
+            for (int j = 0; j < 5; ++j) {
+                const Tensor& x = t[i][j];
+                if (!x.is_cuda() || x.scalar_type() != at::kFloat || !x.is_contiguous() || x.device() != t[0][0].device() ||
+                    x.numel() != (j < 4 ? t[i][0].numel() : 1))
+                    bad("AdamW: contiguous fp32 CUDA tensors of one device are needed");
+                at[j] = x.data_ptr();
+            }
+            where.push_back(at);
+            e.push_back({static_cast<float*>(at[0]), static_cast<const float*>(at[1]), static_cast<float*>(at[2]),
+                         static_cast<float*>(at[3]), static_cast<float*>(at[4]), t[i][0].numel(), int32_t(groups[i]), 0});
+            chunks += (e.back().n + SD_ADAMW_CHUNK - 1) / SD_ADAMW_CHUNK;
+        }
+        const int n = int(e.size());
+        std::vector<char> host(sd_adamw_table_bytes(e.data(), n));
+        check_rc(sd_adamw_table_fill(host.data(), e.data(), n));
+        table = at::from_blob(host.data(), {int64_t(host.size())}, at::kByte).to(t[0][0].device());
+    }
+    // false, with nothing done, if a tensor is no longer where the table says
+    bool step(const std::vector<double>& hyper) {
+        py::gil_scoped_release no_gil;
+        for (size_t i = 0; i < tensors.size(); ++i)
+            for (int j = 0; j < 5; ++j)
+                if (tensors[i][j].data_ptr() != where[i][j]) return false;
+        const at::Device dev = table.device();
+        c10::cuda::OptionalCUDAGuard guard(dev);
+        check_rc(sd_adamw_step(table.data_ptr(), chunks, hyper.data(), int(hyper.size() / 5),
+                               c10::cuda::getCurrentCUDAStream(dev.index()).stream()));
+        for (auto& t : tensors)                    // in-place updates, as autograd sees them
+            for (int j : {0, 2, 3, 4}) t[j].unsafeGetTensorImpl()->bump_version();
+        return true;
+    }
+};
+
 }  // namespace
 
 PYBIND11_MODULE(sd_torch, m) {
@@ -580,10 +827,14 @@ PYBIND11_MODULE(sd_torch, m) {
     });
     register_node();
     m.def("linear", &linear);
+    m.def("conv2d", &conv2d);
     m.def("gemm", &gemm_dense);
     m.def("gemm_dsd", &gemm_dsd);
     m.def("gemm_sdd", &gemm_sdd);
     m.def("layer_norm", &layer_norm);
+    py::class_<AdamW>(m, "AdamW")
+        .def(py::init<const std::vector<std::array<Tensor, 5>>&, const std::vector<int64_t>&>())
+        .def("step", &AdamW::step);
     m.def("status_word", [](int dev) { return status_tensor(dev); });
     m.def("has_status_word", [](int dev) {
         std::lock_guard<std::mutex> lock(state_mutex());

@@ -25,11 +25,13 @@ EXPORTS = (
     "sd_version", "sd_last_error", "sd_plan_bytes", "sd_plan_offsets", "sd_plan_from_seed", "sd_plan_from_seed_counter",
     "sd_plan_from_mask", "sd_workspace_bytes", "sd_workspace_init", "sd_gemm", "sd_gemm_dsd", "sd_gemm_sdd", "sd_gemm_sdd_kept", "sd_gemm_sdd_kept_t",
     "sd_gemm_dsd_static_scratch", "sd_im2col_kept", "sd_col2im_kept", "sd_im2col_kept_panels", "sd_col2im_kept_panels",
+    "sd_col2im_kept_panels_f32",
     "sd_gemm_dsd_panels", "sd_gemm_sdd_kept_t_panels", "sd_selftest_bounded_wait", "sd_check_status",
     "sd_conv_fused_supported", "sd_conv_dsd_fwd", "sd_conv_dsd_dw",
     "sd_gemm_dsd_relu", "sd_gemm_dsd_f32", "sd_gemm_sdd_relu_mask", "sd_gemm_sdd_f32", "sd_cast16",
     "sd_plan_batch_desc_bytes", "sd_plan_batch_describe", "sd_plan_batch_launch", "sd_set_sm_margin",
     "sd_layernorm_fwd", "sd_layernorm_bwd_workspace_bytes", "sd_layernorm_bwd",
+    "sd_adamw_table_bytes", "sd_adamw_table_fill", "sd_adamw_step",
 )
 
 
@@ -90,6 +92,8 @@ def lib() -> C.CDLL:
     L.sd_im2col_kept_panels.argtypes = [vp] + [i32] * 12 + [vp, i32, vp, vp]
     L.sd_col2im_kept_panels.restype = i32
     L.sd_col2im_kept_panels.argtypes = [vp, i32] + [i32] * 12 + [vp, vp, i32, vp]
+    L.sd_col2im_kept_panels_f32.restype = i32
+    L.sd_col2im_kept_panels_f32.argtypes = L.sd_col2im_kept_panels.argtypes
     L.sd_gemm_dsd_panels.restype = i32
     L.sd_gemm_dsd_panels.argtypes = [vp, i32, i32] + mat * 2 + [i32, vp, i32, f32, i32, vp, vp, vp]
     L.sd_gemm_sdd_kept_t_panels.restype = i32

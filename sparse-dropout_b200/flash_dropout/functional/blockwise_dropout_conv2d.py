@@ -14,6 +14,7 @@ colP[ceil(M/128)][K64][128], so that every kept 128x128 block is one contiguous 
   backward  DSD          : dW2d[Kout, K] written transposed, reduction over kept row blocks of each K tile
             SDD          : kept blocks of dcolP = W2d^T . dy2d^T / (1-p)         (plan of the transposed result)
             col2im_kept  : dx (NCHW) = adjoint gather over kept blocks           (HBM-bound)
+The launches and the autograd node are native code (csrc/sd_torch.cpp: conv2d, SparseDropConv2dBackward).
   By default the kept blocks of colT are saved for backward (151 MB for a 256x64x32x32 input with a 3x3 filter, half of what an
   unfold-based layer keeps); ``recompute_cols=True`` saves only the input (33 MB) and rebuilds colT in backward.
 """
@@ -25,8 +26,7 @@ import torch
 
 from flash_dropout import _lib
 from flash_dropout import random as sd_random
-from flash_dropout.cuda.binding_gemm import (BlockPlan, _on_device, conv_dsd_dw, conv_dsd_fwd, conv_fused_supported,
-                                             dsd_panels, sdd_kept_t_panels)
+from flash_dropout.cuda.binding_gemm import BlockPlan, PlanBatch, _on_device, _rep
 
 from .blockwise_dropout_matmul_cuda import _autocast_input
 from .im2col_conv2d import conv_output_size
@@ -97,77 +97,6 @@ def col2im_kept(dcolT: torch.Tensor, x_shape, kernel_size, padding, stride, dila
     return dx
 
 
-class BlockwiseDropoutConv2dCUDA(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, input, kernel, block_size, p, padding, stride, dilation, plan, recompute_cols, fused):
-        assert 0 <= p < 1, "Dropout probability must be in [0, 1)"
-        if not (input.is_cuda and kernel.is_cuda):
-            raise RuntimeError("input and kernel must be CUDA")
-        if input.dtype != kernel.dtype:
-            raise RuntimeError(f"input ({input.dtype}) and kernel ({kernel.dtype}) must have the same dtype")
-        _lib.dtype_code(input.dtype)
-        N, C, H, W = input.shape
-        Ko, Ck, R, S = kernel.shape
-        if Ck != C:
-            raise RuntimeError(f"kernel expects {Ck} input channels, input has {C}")
-        P, Q = conv_output_size(H, W, R, S, padding, stride, dilation)
-        M, K = N * P * Q, C * R * S
-        Kg, Kog = _round64(K), _round8(Ko)       # the im2col matrix is kept in panels: k extent a multiple of 64
-        if plan is None:
-            plan = BlockPlan.draw(M, Kg, block_size, p, input.device)
-        w2d = kernel.reshape(Ko, K)
-        if Kg != K or Kog != Ko:                         # 16-byte rows for TMA; zero padding changes nothing
-            w2d = torch.nn.functional.pad(w2d, (0, Kg - K, 0, Kog - Ko))
-        w2d = w2d.contiguous()
-        input = input.contiguous()
-        ctx.fused = fused and conv_fused_supported(input.shape, (R, S), padding, stride, dilation)
-        if ctx.fused:
-            # im2col + DSD in one kernel: the matrix is gathered stage by stage from the input, never stored
-            y2d = conv_dsd_fwd(input, w2d, plan, (R, S), padding, stride, dilation, 1.0 / (1.0 - p))   # (M, Kog)
-            ctx.save_for_backward(input, w2d)
-        else:
-            colT = im2col_kept(input, (R, S), padding, stride, dilation, plan, Kg, panels=True)
-            y2d = dsd_panels(colT, M, w2d, plan, _lib.SD_PLAN_ROWS, 1.0 / (1.0 - p))   # (M, Kog)
-            if recompute_cols:
-                ctx.save_for_backward(input, w2d)
-            else:
-                ctx.save_for_backward(input, w2d, colT)
-        ctx.plan, ctx.p = plan, p
-        ctx.geom = (padding, stride, dilation, (R, S), Ko, K)
-        return y2d.view(N, P, Q, Kog)[..., :Ko].permute(0, 3, 1, 2)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        input, w2d, *saved_cols = ctx.saved_tensors
-        plan, scale = ctx.plan, 1.0 / (1.0 - ctx.p)
-        padding, stride, dilation, (R, S), Ko, K = ctx.geom
-        N, C, H, W = input.shape
-        Kog, Kg = w2d.shape
-        M = grad_output.numel() // Ko
-        dy2d = grad_output.to(input.dtype).permute(0, 2, 3, 1).reshape(M, Ko)   # free for channels_last gradients
-        if Kog != Ko:
-            dy2d = torch.nn.functional.pad(dy2d, (0, Kog - Ko))
-        dy2d = dy2d.contiguous()
-        grad_input = grad_kernel = None
-        if ctx.needs_input_grad[1] and ctx.fused:
-            dw2d = torch.empty((Kog, Kg), dtype=input.dtype, device=input.device)
-            conv_dsd_dw(input, dy2d, plan, (R, S), padding, stride, dilation, scale, out=dw2d)
-            grad_kernel = dw2d[:Ko, :K].reshape(Ko, C, R, S)
-        elif ctx.needs_input_grad[1]:
-            colT = saved_cols[0] if saved_cols else im2col_kept(input, (R, S), padding, stride, dilation, plan, Kg,
-                                                                 panels=True)
-            dw2d = torch.empty((Kog, Kg), dtype=input.dtype, device=input.device)
-            dsd_panels(colT, M, dy2d.T, plan, _lib.SD_PLAN_COLS, scale, out=dw2d.T)
-            grad_kernel = dw2d[:Ko, :K].reshape(Ko, C, R, S)
-            del colT
-        if ctx.needs_input_grad[0]:
-            dcolT = torch.empty((ceil(M / 128), Kg, 128), dtype=input.dtype, device=input.device)
-            # dcolT = w2d.T @ dy2d.T on the kept blocks, written into panels; col2im reads kept blocks only
-            sdd_kept_t_panels(w2d.T, dy2d, plan, scale, out=dcolT)
-            grad_input = col2im_kept(dcolT, input.shape, (R, S), padding, stride, dilation, plan)
-        return grad_input, grad_kernel, None, None, None, None, None, None, None, None
-
-
 def blockwise_dropout_conv2d(input: torch.Tensor, kernel: torch.Tensor, block_size: int, p: float,
                              padding=(0, 0), stride=(1, 1), dilation=(1, 1), plan=None,
                              recompute_cols: bool = False, fused: bool = True) -> torch.Tensor:
@@ -176,9 +105,32 @@ def blockwise_dropout_conv2d(input: torch.Tensor, kernel: torch.Tensor, block_si
     ``fused`` (default): geometries the fused kernels serve (3-wide filters, unit horizontal stride / dilation, one
     column of padding, rows of 8..64 pixels) never materialise the im2col matrix; others, and ``fused=False``, go
     through the kept-block im2col stage."""
+    assert 0 <= p < 1, "Dropout probability must be in [0, 1)"
     if torch.is_autocast_enabled("cuda"):
+        # fp32 tensors are cast inside the operator and get their gradients in fp32; others by autograd
         dt = torch.get_autocast_dtype("cuda")
-        input, kernel = _autocast_input(input, dt), kernel.to(dt)
-    with torch.autocast("cuda", enabled=False):
-        return BlockwiseDropoutConv2dCUDA.apply(input, kernel, block_size, p, tuple(padding), tuple(stride),
-                                                tuple(dilation), plan, recompute_cols, fused)
+        if input.dtype not in (dt, torch.float32):
+            input = _autocast_input(input, dt)
+        if kernel.dtype not in (dt, torch.float32):
+            kernel = kernel.to(dt)
+    padding, stride, dilation = tuple(padding), tuple(stride), tuple(dilation)
+    seed = offset = 0
+    counter = None
+    fresh = False
+    if plan is None:
+        if PlanBatch.active is not None:
+            N, C, H, W = input.shape
+            R, S = kernel.shape[2:]
+            P, Q = conv_output_size(H, W, R, S, padding, stride, dilation)
+            plan = BlockPlan.draw(N * P * Q, _round64(C * R * S), block_size, p, input.device)
+        elif input.is_cuda and (counter := sd_random.device_counter(input.device)) is not None:
+            seed, offset = sd_random.seed_and_base()
+        else:
+            seed, offset = sd_random.peek_seed_offset()
+            fresh = True
+    buf, R, C = (None, 0, 0) if plan is None else (plan.buf, plan.R, plan.C)
+    out = _lib.ext().conv2d(input, kernel, buf, R, C, *_rep(block_size), p, seed, offset, counter, padding, stride, dilation,
+                            recompute_cols, fused)
+    if fresh:
+        sd_random.advance()                    # the mask has been drawn; a call that raised has used none
+    return out

@@ -50,7 +50,7 @@ def _autocast_input(input: torch.Tensor, dt: torch.dtype) -> torch.Tensor:
 def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_size: int, p: float,
                              plan: BlockPlan | None = None, relu: bool = False, input_relu: bool = False,
                              grad_premasked: bool = False, wgrad=None, recompute_plan: bool = False,
-                             weight_lowp: torch.Tensor | None = None) -> torch.Tensor:
+                             weight_lowp: torch.Tensor | None = None, any_rank: bool = False) -> torch.Tensor:
     """``y = (mask o input) . weight^T / (1 - p)`` with a fresh block mask (or the given plan).
 
     Under CUDA autocast both operands are cast to the autocast dtype (the reference casts to fp16,
@@ -72,7 +72,8 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
                       from the device-side counter (CUDA-graph mode, where plan buffers are static anyway) is kept;
       weight_lowp     an up-to-date copy of ``weight`` in the autocast dtype that the caller keeps (a training step that
                       casts all weights with one launch): used instead of casting again, which needs ``wgrad`` (the copy
-                      is outside autograd, so the weight gradient has to leave through the fused store).
+                      is outside autograd, so the weight gradient has to leave through the fused store);
+      any_rank        ``input`` may have any number of leading dimensions, all of them rows.
     """
     assert 0 <= p < 1, "Dropout probability must be in [0, 1)"
     rep_r, rep_c = _rep(block_size)
@@ -81,8 +82,8 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
     fresh = False
     if plan is None:
         if PlanBatch.active is not None:
-            M, K = input.shape
-            plan = BlockPlan.draw(M, K, block_size, p, input.device)
+            K = input.shape[-1]
+            plan = BlockPlan.draw(input.numel() // K, K, block_size, p, input.device)
         elif input.is_cuda and (counter := sd_random.device_counter(input.device)) is not None:
             seed, offset = sd_random.seed_and_base()
         else:
@@ -96,10 +97,15 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
             seed, offset = plan.origin[4:]
         else:
             recompute_plan = False
+    if torch.is_autocast_enabled("cuda"):
+        # fp32 operands are cast inside the operator; others by autograd
+        dt = torch.get_autocast_dtype("cuda")
+        if input.dtype not in (dt, torch.float32):
+            input = _autocast_input(input, dt)
     target, accumulate, notify = wgrad if wgrad is not None else (None, False, None)
     out = _lib.ext().linear(input, weight, buf, R, C, rep_r, rep_c, not isinstance(block_size, int), p, seed, offset,
                             counter, relu, input_relu, grad_premasked, target, accumulate, notify, recompute_plan,
-                            weight_lowp)
+                            weight_lowp, any_rank)
     if fresh:
         sd_random.advance()                    # the mask has been drawn; a call that raised has used none
     return out

@@ -55,17 +55,16 @@ class DropoutMM(nn.Module):
             raise ValueError(f"Unknown activation {activation}")
         v = self.variant
         if self.training and v in ("blockwise[cuda]", "blockwise[triton]"):
-            lead = input.shape[:-1]
-            x = input.reshape(-1, input.shape[-1])
-            wgrad = getattr(self.weight, "_sd_wgrad", None) if torch.is_grad_enabled() else None
+            weight = self.weight
+            wgrad = getattr(weight, "_sd_wgrad", None) if torch.is_grad_enabled() else None
             # a 16-bit copy of the weight kept by the training step, valid while the weight has not changed since
-            lowp = getattr(self.weight, "_sd_w16", None)
-            lowp = lowp[0] if (lowp is not None and wgrad is not None and lowp[1] == self.weight._version) else None
-            out = F.cuda_blockwise_dropout_matmul(x, self.weight, _block_size(self.kwargs), self.p, weight_lowp=lowp,
-                                                  relu=activation == "relu", input_relu=input_relu,
-                                                  grad_premasked=grad_premasked and activation == "relu", wgrad=wgrad,
-                                                  recompute_plan=bool(self.kwargs.get("recompute_plan", False)))
-            return out.reshape(*lead, self.out_features)
+            lowp = getattr(weight, "_sd_w16", None) if wgrad is not None else None
+            lowp = lowp[0] if (lowp is not None and lowp[1] == weight._version) else None
+            return F.cuda_blockwise_dropout_matmul(input, weight, _block_size(self.kwargs), self.p, weight_lowp=lowp,
+                                                   relu=activation == "relu", input_relu=input_relu,
+                                                   grad_premasked=grad_premasked and activation == "relu", wgrad=wgrad,
+                                                   recompute_plan=bool(self.kwargs.get("recompute_plan", False)),
+                                                   any_rank=True)
         out = self._forward_plain(input)
         return torch.relu(out) if activation == "relu" else out
 
@@ -81,8 +80,6 @@ class DropoutMM(nn.Module):
             out = F.vanilla_dropout_matmul(x, self.weight, self.p)
         elif v == "blockwise[naive]":
             out = F.naive_blockwise_dropout_matmul(x, self.weight, _block_size(self.kwargs), self.p)
-        elif v in ("blockwise[cuda]", "blockwise[triton]"):
-            out = F.cuda_blockwise_dropout_matmul(x, self.weight, _block_size(self.kwargs), self.p)
         else:
             raise ValueError(f"Unknown variant {v}")
         return out.reshape(*lead, self.out_features)
