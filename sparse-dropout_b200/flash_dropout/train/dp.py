@@ -20,6 +20,8 @@ import os
 import torch
 import torch.distributed as dist
 
+from torch.optim import optimizer as _torch_optimizer
+
 from flash_dropout import random as sd_random
 
 
@@ -77,6 +79,7 @@ class FlatGradDataParallel:
                     dist.broadcast(b.data, src=broadcast_from, group=self.group)
             for p in self.params:
                 p.register_post_accumulate_grad_hook(self._on_grad_ready)
+        self.adamw = _FusedAdamW()
         self._shadow_params: list = []
         self._shadows = None
         if fuse_wgrad:
@@ -208,6 +211,86 @@ class FlatGradDataParallel:
         return all(p.grad is not None and p.grad.data_ptr() == base + self._esize * self._slices[p][0] for p in self.params)
 
 
+class _FusedAdamW:
+    """``optimizer.step()`` of a plain ``torch.optim.AdamW`` as one launch of this library's kernel (``sd_adamw_step``).
+
+    It updates the optimizer's own state tensors in place, so ``state_dict()``, checkpoints and a later ``optimizer.step()``
+    see nothing unusual.  Anything the kernel does not do (AMSGrad, maximize, tensor learning rates, step counters on the
+    host, hooks, a patched ``step``, a gradient scaler, parameters without a gradient) and the first step, which creates
+    the state, are left to the optimizer itself.  The description of the tensors is made once and checked at every step."""
+
+    MAX_GROUPS = 8                                     # SD_ADAMW_MAX_GROUPS
+
+    def __init__(self):
+        self._native = None
+        self._seen: list = []                          # (parameter, gradient, state, exp_avg, exp_avg_sq, step)
+
+    @staticmethod
+    def _plain(optimizer) -> bool:
+        if type(optimizer) is not torch.optim.AdamW or "step" in optimizer.__dict__ or hasattr(optimizer, "grad_scale"):
+            return False
+        if optimizer._optimizer_step_pre_hooks or optimizer._optimizer_step_post_hooks:
+            return False
+        if _torch_optimizer._global_optimizer_pre_hooks or _torch_optimizer._global_optimizer_post_hooks:
+            return False
+        groups = optimizer.param_groups
+        return len(groups) <= _FusedAdamW.MAX_GROUPS and not any(
+            g["amsgrad"] or g["maximize"] or g["differentiable"] or not isinstance(g["lr"], (int, float))
+            or not all(isinstance(b, (int, float)) for b in g["betas"]) for g in groups)
+
+    def _current(self, optimizer) -> bool:
+        if sum(len(g["params"]) for g in optimizer.param_groups) != len(self._seen):
+            return False
+        state, i = optimizer.state, 0
+        for group in optimizer.param_groups:
+            for p in group["params"]:
+                q, grad, st, m, v, step = self._seen[i]
+                i += 1
+                if p is not q or p.grad is not grad or state.get(p) is not st:
+                    return False
+                if st["exp_avg"] is not m or st["exp_avg_sq"] is not v or st["step"] is not step:
+                    return False
+        return True
+
+    def _describe(self, optimizer) -> bool:
+        self._native, self._seen = None, []
+        seen, tensors, groups = [], [], []
+        device = optimizer.param_groups[0]["params"][0].device
+        for i, group in enumerate(optimizer.param_groups):
+            for p in group["params"]:
+                st = optimizer.state.get(p)
+                if p.grad is None or not st or "step" not in st:
+                    return False
+                entry = (p, p.grad, st["exp_avg"], st["exp_avg_sq"], st["step"])
+                if not all(isinstance(t, torch.Tensor) and t.layout == torch.strided and t.is_cuda and t.dtype == torch.float32
+                           and t.is_contiguous() and t.device == device for t in entry):
+                    return False
+                if st["step"].numel() != 1 or any(t.data_ptr() % 16 for t in entry[:4]):
+                    return False
+                seen.append((p, p.grad, st, *entry[2:]))
+                tensors.append(list(entry))
+                groups.append(i)
+        if not seen:
+            return False
+        from flash_dropout import _lib
+        self._native = _lib.ext().AdamW(tensors, groups)
+        self._seen = seen
+        return True
+
+    def step(self, optimizer) -> None:
+        if self._plain(optimizer):
+            if self._native is not None and not self._current(optimizer):
+                self._native = None
+            if self._native is not None or (torch.cuda.is_available() and not torch.cuda.is_current_stream_capturing()
+                                            and self._describe(optimizer)):
+                hyper = []
+                for g in optimizer.param_groups:
+                    hyper += (g["lr"], *g["betas"], g["eps"], g["weight_decay"])
+                if self._native.step(hyper):
+                    return
+        optimizer.step()
+
+
 _steps_since_check = 0
 
 
@@ -242,7 +325,7 @@ def train_step(model: torch.nn.Module, dp: FlatGradDataParallel, optimizer: torc
         loss = loss_fn(model)
     loss.backward()
     dp.finish()
-    optimizer.step()
+    dp.adamw.step(optimizer)
     return loss.detach()
 
 
@@ -301,7 +384,7 @@ class GraphedTrainStep:
             loss.backward()
             if self.whole_step:
                 dp.finish()
-                optimizer.step()
+                dp.adamw.step(optimizer)
             return loss.detach()
 
         def fwd_loss():
@@ -322,6 +405,7 @@ class GraphedTrainStep:
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph, capture_error_mode="thread_local"):
             self.loss = fwd_bwd()
+        self._adamw_table = dp.adamw._native            # the captured update reads it at every replay
 
     @staticmethod
     def _make_capturable(optimizer: torch.optim.Optimizer) -> bool:

@@ -1,0 +1,59 @@
+"""The one-launch AdamW of the training steps against torch's own optimizer."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("sizes", [[1], [2047, 2048, 2049], [5, 3, 4096 * 3 + 1, 300_003]])
+@pytest.mark.parametrize("capturable", [False, True])
+def test_adamw_matches_torch(built_lib, sizes, capturable):
+    """Five steps with two parameter groups and changing gradients and learning rate.  Both sides evaluate the same formula
+    in fp32; the few roundings per step that may fall differently move a parameter by at most ~4 ulp of its update
+    (4 * 2^-23 * lr per step), far below the bound, and the moments by ulps."""
+    from flash_dropout.train.dp import _FusedAdamW
+    g = torch.Generator().manual_seed(sum(sizes))
+    start = [torch.randn(n, generator=g) for n in sizes]
+    grads = [[torch.randn(n, generator=g) * 10.0 ** -k for n in sizes] for k in range(5)]
+    sides = []
+    for ours in (False, True):
+        params = [torch.nn.Parameter(t.to(DEV)) for t in start]
+        groups = [{"params": params[:1], "weight_decay": 0.1}, {"params": params[1:], "weight_decay": 0.0}]
+        opt = torch.optim.AdamW([gr for gr in groups if gr["params"]], lr=1e-2, fused=True, capturable=capturable)
+        # every gradient 16-byte aligned, as the kernel asks; a misaligned one takes torch's step
+        for p in params:
+            p.grad = torch.zeros_like(p)
+        fused = _FusedAdamW()
+        for k in range(5):
+            for gr in opt.param_groups:
+                gr["lr"] = 1e-2 / (k + 1)
+            for p, t in zip(params, grads[k]):
+                p.grad.copy_(t)
+            fused.step(opt) if ours else opt.step()
+        assert not ours or fused._native is not None
+        sides.append([(p.detach(), *(opt.state[p][k] for k in ("exp_avg", "exp_avg_sq", "step"))) for p in params])
+    for a, b in zip(*sides):
+        assert torch.equal(a[3], b[3]) and a[3].item() == 5
+        for x, y in zip(a[:3], b[:3]):
+            torch.testing.assert_close(x, y, rtol=1e-5, atol=1e-7)
+
+
+def test_anything_else_is_left_to_the_optimizer(built_lib):
+    from flash_dropout.train.dp import _FusedAdamW
+    p = torch.nn.Parameter(torch.ones(8, device=DEV))
+    p.grad = torch.ones_like(p)
+    for make in (lambda: torch.optim.AdamW([p], amsgrad=True), lambda: torch.optim.Adam([p]), lambda: torch.optim.SGD([p], lr=0.1)):
+        opt, fused = make(), _FusedAdamW()
+        before = p.detach().clone()
+        for _ in range(2):
+            fused.step(opt)
+        assert fused._native is None and not torch.equal(before, p)
+    opt, fused = torch.optim.AdamW([p], lr=0.1, fused=True), _FusedAdamW()
+    for _ in range(2):
+        fused.step(opt)
+    assert fused._native is not None
+    opt.load_state_dict(opt.state_dict())                  # new state tensors: described again, not updated through stale pointers
+    steps = opt.state[p]["step"]
+    fused.step(opt)
+    assert steps.item() == 3
