@@ -51,6 +51,36 @@ inline void check_rc(int rc) {
 }
 [[noreturn]] inline void bad(const std::string& msg) { throw std::runtime_error(msg); }
 
+// The Python error that is set (GIL held), as the exception that autograd's engine carries from its threads to the caller
+// of backward() with its type; any other exception arrives there as a plain RuntimeError.
+[[noreturn]] void throw_python() {
+    python_error e;
+    e.persist();
+    throw std::move(e);
+}
+void set_python_error(const SdError& err) {
+    static PyObject* type = py::module_::import("flash_dropout._lib").attr("SparseDropError").cast<py::object>().release().ptr();
+    PyErr_SetString(type, err.what());
+}
+// The body of a node's apply().
+template <class F>
+variable_list backward_call(F&& body) {
+    try {
+        return body();
+    } catch (const SdError& err) {
+        py::gil_scoped_acquire gil;
+        set_python_error(err);
+        throw_python();
+    }
+}
+
+// These nodes have no forward-mode derivative: a dual tensor is refused, as by a torch.autograd.Function without a jvp.
+void no_forward_ad(const char* what, std::initializer_list<std::reference_wrapper<const Tensor>> inputs) {
+    for (const Tensor& t : inputs)
+        if (torch::autograd::isFwGradDefined(t))
+            bad(std::string("Trying to use forward AD with ") + what + " that does not support it because it has not been implemented yet.");
+}
+
 int dtype_code(at::ScalarType t) {
     if (t == at::kHalf) return SD_F16;
     if (t == at::kBFloat16) return SD_BF16;
@@ -769,14 +799,16 @@ std::optional<Tensor> layer_norm(const Tensor& x, const Tensor& weight, const st
 }
 
 // ---------------------------------------------------------------- AdamW
-// The tensors of one optimizer, described to the kernel once; a step checks that none of them has moved since.
+// The tensors of one optimizer, described to the kernel once; a step checks that none of them has moved since.  Only weak
+// references are held: parameters lead back to whoever holds this object (their gradient hooks), and Python's collector
+// cannot look through it.
 struct AdamW {
-    std::vector<std::array<Tensor, 5>> tensors;    // p, g, m, v, step
+    std::vector<std::array<c10::weak_intrusive_ptr<c10::TensorImpl>, 5>> tensors;    // p, g, m, v, step
     std::vector<std::array<void*, 5>> where;
     Tensor table;
     int64_t chunks = 0;
 
-    AdamW(const std::vector<std::array<Tensor, 5>>& t, const std::vector<int64_t>& groups) : tensors(t) {
+    AdamW(const std::vector<std::array<Tensor, 5>>& t, const std::vector<int64_t>& groups) {
         std::vector<sd_adamw_entry> e;
         for (size_t i = 0; i < t.size(); ++i) {
             std::array<void*, 5> at;
@@ -788,6 +820,9 @@ struct AdamW {
                 at[j] = x.data_ptr();
             }
             where.push_back(at);
+            using Weak = c10::weak_intrusive_ptr<c10::TensorImpl>;
+            tensors.push_back({Weak(t[i][0].getIntrusivePtr()), Weak(t[i][1].getIntrusivePtr()), Weak(t[i][2].getIntrusivePtr()),
+                               Weak(t[i][3].getIntrusivePtr()), Weak(t[i][4].getIntrusivePtr())});
             e.push_back({static_cast<float*>(at[0]), static_cast<const float*>(at[1]), static_cast<float*>(at[2]),
                          static_cast<float*>(at[3]), static_cast<float*>(at[4]), t[i][0].numel(), int32_t(groups[i]), 0});
             chunks += (e.back().n + SD_ADAMW_CHUNK - 1) / SD_ADAMW_CHUNK;
@@ -797,18 +832,24 @@ struct AdamW {
         check_rc(sd_adamw_table_fill(host.data(), e.data(), n));
         table = at::from_blob(host.data(), {int64_t(host.size())}, at::kByte).to(t[0][0].device());
     }
-    // false, with nothing done, if a tensor is no longer where the table says
+    // false, with nothing done, if a tensor is gone or no longer where the table says
     bool step(const std::vector<double>& hyper) {
         py::gil_scoped_release no_gil;
+        std::vector<Tensor> held;
+        held.reserve(5 * tensors.size());
         for (size_t i = 0; i < tensors.size(); ++i)
-            for (int j = 0; j < 5; ++j)
-                if (tensors[i][j].data_ptr() != where[i][j]) return false;
+            for (int j = 0; j < 5; ++j) {
+                auto t = tensors[i][j].lock();
+                if (!t) return false;
+                held.emplace_back(std::move(t));
+                if (held.back().data_ptr() != where[i][j]) return false;
+            }
         const at::Device dev = table.device();
         c10::cuda::OptionalCUDAGuard guard(dev);
         check_rc(sd_adamw_step(table.data_ptr(), chunks, hyper.data(), int(hyper.size() / 5),
                                c10::cuda::getCurrentCUDAStream(dev.index()).stream()));
-        for (auto& t : tensors)                    // in-place updates, as autograd sees them
-            for (int j : {0, 2, 3, 4}) t[j].unsafeGetTensorImpl()->bump_version();
+        for (size_t i = 0; i < held.size(); ++i)   // in-place updates, as autograd sees them
+            if (i % 5 != 1) held[i].unsafeGetTensorImpl()->bump_version();
         return true;
     }
 };

@@ -57,3 +57,21 @@ def test_anything_else_is_left_to_the_optimizer(built_lib):
     steps = opt.state[p]["step"]
     fused.step(opt)
     assert steps.item() == 3
+
+
+def test_a_model_that_has_been_stepped_is_freed(built_lib):
+    """The optimizer's description must not keep parameters alive: they lead back to it through their gradient hooks."""
+    import gc
+    import weakref
+    from flash_dropout.train import BasicNet, FlatGradDataParallel, train_step
+    model = BasicNet(128, 2, 128, 10, dict(p=0.5, variant="blockwise[cuda]", block_size=128)).to(DEV)
+    dp = FlatGradDataParallel(model)
+    opt = torch.optim.AdamW(model.parameters(), lr=1e-3, fused=True)
+    x = torch.randn(128, 128, device=DEV)
+    for _ in range(3):
+        train_step(model, dp, opt, lambda m: m(x).square().mean(), autocast_dtype=torch.bfloat16)
+    assert dp.adamw._native is not None
+    gone = [weakref.ref(dp), weakref.ref(model)]
+    del model, dp, opt
+    gc.collect()
+    assert all(r() is None for r in gone)
