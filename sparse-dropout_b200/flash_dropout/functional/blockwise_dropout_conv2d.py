@@ -126,11 +126,13 @@ def blockwise_dropout_conv2d(input: torch.Tensor, kernel: torch.Tensor, block_si
         elif input.is_cuda and (counter := sd_random.device_counter(input.device)) is not None:
             seed, offset = sd_random.seed_and_base()
         else:
-            seed, offset = sd_random.peek_seed_offset()
+            seed, offset = sd_random.next_seed_offset()
             fresh = True
     buf, R, C = (None, 0, 0) if plan is None else (plan.buf, plan.R, plan.C)
-    out = _lib.ext().conv2d(input, kernel, buf, R, C, *_rep(block_size), p, seed, offset, counter, padding, stride, dilation,
-                            recompute_cols, fused)
-    if fresh:
-        sd_random.advance()                    # the mask has been drawn; a call that raised has used none
-    return out
+    try:
+        return _lib.ext().conv2d(input, kernel, buf, R, C, *_rep(block_size), p, seed, offset, counter, padding, stride, dilation,
+                                recompute_cols, fused)
+    except Exception:
+        if fresh:
+            sd_random.give_back(offset)        # a call that was refused has used no mask
+        raise

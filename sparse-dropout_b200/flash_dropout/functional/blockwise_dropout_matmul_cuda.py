@@ -87,7 +87,7 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
         elif input.is_cuda and (counter := sd_random.device_counter(input.device)) is not None:
             seed, offset = sd_random.seed_and_base()
         else:
-            seed, offset = sd_random.peek_seed_offset()
+            seed, offset = sd_random.next_seed_offset()
             fresh = True
     if plan is None:
         buf, R, C = None, 0, 0
@@ -103,12 +103,14 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
         if input.dtype not in (dt, torch.float32):
             input = _autocast_input(input, dt)
     target, accumulate, notify = wgrad if wgrad is not None else (None, False, None)
-    out = _lib.ext().linear(input, weight, buf, R, C, rep_r, rep_c, not isinstance(block_size, int), p, seed, offset,
-                            counter, relu, input_relu, grad_premasked, target, accumulate, notify, recompute_plan,
-                            weight_lowp, any_rank)
-    if fresh:
-        sd_random.advance()                    # the mask has been drawn; a call that raised has used none
-    return out
+    try:
+        return _lib.ext().linear(input, weight, buf, R, C, rep_r, rep_c, not isinstance(block_size, int), p, seed, offset,
+                                counter, relu, input_relu, grad_premasked, target, accumulate, notify, recompute_plan,
+                                weight_lowp, any_rank)
+    except Exception:
+        if fresh:
+            sd_random.give_back(offset)        # a call that was refused has used no mask
+        raise
 
 
 class BlockwiseDropoutMatmulCUDA:

@@ -8,11 +8,14 @@ selects a disjoint range of offsets so that ranks draw different masks from one 
 """
 from __future__ import annotations
 
+import threading
+
 import torch
 
 _state = {"seed": None, "torch_seed": None, "offset": 0, "subsequence": 0}
 _device_counters: dict = {}      # device index -> uint64 CUDA tensor holding the offset counter
 _SUBSEQ_SHIFT = 40
+_lock = threading.Lock()
 
 
 def manual_seed(seed: int, subsequence: int | None = None) -> None:
@@ -43,29 +46,28 @@ def set_state(state: dict) -> None:
     _state.update(state)
 
 
-def peek_seed_offset() -> tuple[int, int]:
-    """(seed, offset) for the next mask."""
-    if _state["seed"] is None:
-        ts = torch.initial_seed()
-        if ts != _state["torch_seed"]:
-            _state["torch_seed"] = ts
-            _state["offset"] = 0
-        seed = ts
-    else:
-        seed = _state["seed"]
-    return seed & (2**64 - 1), (_state["subsequence"] << _SUBSEQ_SHIFT) + _state["offset"]
-
-
-def advance() -> None:
-    """Moves on to the following mask."""
-    _state["offset"] += 1
-
-
 def next_seed_offset() -> tuple[int, int]:
-    """(seed, offset) for the next mask; advances the counter."""
-    out = peek_seed_offset()
-    advance()
-    return out
+    """(seed, offset) for the next mask; advances the counter.  Calls from several threads get different offsets."""
+    with _lock:
+        if _state["seed"] is None:
+            ts = torch.initial_seed()
+            if ts != _state["torch_seed"]:
+                _state["torch_seed"] = ts
+                _state["offset"] = 0
+            seed = ts
+        else:
+            seed = _state["seed"]
+        off = _state["offset"]
+        _state["offset"] = off + 1
+        return seed & (2**64 - 1), (_state["subsequence"] << _SUBSEQ_SHIFT) + off
+
+
+def give_back(offset: int) -> None:
+    """The mask at ``offset`` was not drawn after all (the call was refused): the next call gets it, unless another thread
+    has moved on."""
+    with _lock:
+        if (_state["subsequence"] << _SUBSEQ_SHIFT) + _state["offset"] == offset + 1:
+            _state["offset"] -= 1
 
 
 def enable_device_counter(device: torch.device, start: int = 0) -> torch.Tensor:

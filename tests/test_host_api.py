@@ -206,3 +206,54 @@ def test_layernorm_module_is_torch_layernorm_on_cpu():
     ref.load_state_dict(ours.state_dict())
     x = torch.randn(5, 7, 48)
     assert torch.equal(ours(x), ref(x))
+
+
+def test_masks_drawn_by_several_threads_differ(monkeypatch):
+    """Each call takes its place in the mask sequence before the native code runs (and lets other threads in)."""
+    import threading
+    import time
+    import types
+
+    import flash_dropout.functional as F
+    from flash_dropout import _lib
+    from flash_dropout import random as sd_random
+    taken = []
+
+    def linear(input, weight, buf, R, C, rep_r, rep_c, pair, p, seed, offset, *rest):
+        time.sleep(0.02)
+        taken.append(offset)
+        return input
+
+    monkeypatch.setattr(_lib, "ext", lambda: types.SimpleNamespace(linear=linear))
+    sd_random.manual_seed(1, subsequence=0)
+    try:
+        x = torch.zeros(128, 128)
+        threads = [threading.Thread(target=F.cuda_blockwise_dropout_matmul, args=(x, x, 128, 0.5)) for _ in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert sorted(taken) == [0, 1, 2, 3] and sd_random.next_seed_offset()[1] == 4
+    finally:
+        sd_random.follow_torch_seed()
+
+
+def test_a_refused_call_uses_no_mask(monkeypatch):
+    import types
+
+    import flash_dropout.functional as F
+    from flash_dropout import _lib
+    from flash_dropout import random as sd_random
+
+    def refuse(*args):
+        raise RuntimeError("input and weight must be CUDA")
+
+    monkeypatch.setattr(_lib, "ext", lambda: types.SimpleNamespace(linear=refuse))
+    sd_random.manual_seed(1, subsequence=3)
+    try:
+        with pytest.raises(RuntimeError):
+            F.cuda_blockwise_dropout_matmul(torch.zeros(8, 8), torch.zeros(8, 8), 128, 0.5)
+        assert sd_random.next_seed_offset()[1] == 3 << 40
+    finally:
+        sd_random.manual_seed(0, subsequence=0)
+        sd_random.follow_torch_seed()
