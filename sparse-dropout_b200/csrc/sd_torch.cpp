@@ -342,6 +342,7 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     if (!input_.is_cuda() || !weight_.is_cuda()) bad("input and weight must be CUDA");   // no CPU path, as gemm_binding.cu:19
     if ((any_rank ? input_.dim() < 1 : input_.dim() != 2) || weight_.dim() != 2) bad("input and weight must be 2D");
     if (input_.device() != weight_.device()) bad("A and B must be on the same device");
+    no_forward_ad("SparseDropLinear", {input_, weight_});
     const at::Device dev = input_.device();
     c10::cuda::OptionalCUDAGuard guard(dev);
     const Launch L(dev);
@@ -621,6 +622,7 @@ Tensor conv2d(const Tensor& input_, const Tensor& kernel_, const std::optional<T
               bool want_fused) {
     py::gil_scoped_release no_gil;
     if (!input_.is_cuda() || !kernel_.is_cuda()) bad("input and kernel must be CUDA");
+    no_forward_ad("SparseDropConv2d", {input_, kernel_});
     const Tensor &input = input_, &kernel = kernel_;
     const bool amp = at::autocast::is_autocast_enabled(at::kCUDA);
     const at::ScalarType t = amp ? at::autocast::get_autocast_dtype(at::kCUDA) : input.scalar_type();
@@ -770,6 +772,7 @@ std::optional<Tensor> layer_norm(const Tensor& x, const Tensor& weight, const st
         if (dt == at::kHalf || dt == at::kBFloat16) out_t = dt;
     }
     const Tensor bias = bias_ ? *bias_ : Tensor();
+    no_forward_ad("SparseDropLayerNorm", {x, weight, bias});
     const at::Device dev = x.device();
     c10::cuda::OptionalCUDAGuard guard(dev);
     cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();

@@ -47,3 +47,18 @@ def test_input_gradient_in_fp32(built_lib, M, N, K, masked):
                                          bg.workspace(DEV).data_ptr(), bg.status_word(DEV).data_ptr(),
                                          torch.cuda.current_stream().cuda_stream))
     torch.testing.assert_close(dx.cpu(), want.float(), rtol=1e-3, atol=1e-3)
+
+
+def test_forward_mode_is_refused(built_lib):
+    """No forward derivative is implemented: a dual tensor raises instead of losing its tangent."""
+    import flash_dropout.functional as F
+    import torch.autograd.forward_ad as fwad
+    from flash_dropout.layers.norm import layer_norm
+    x = torch.randn(128, 128, device=DEV, dtype=torch.float16)
+    img = torch.randn(1, 8, 8, 8, device=DEV, dtype=torch.float16)
+    with fwad.dual_level():
+        for call in (lambda: F.cuda_blockwise_dropout_matmul(fwad.make_dual(x, x), x, 128, 0.5),
+                     lambda: F.cuda_blockwise_dropout_conv2d(fwad.make_dual(img, img), torch.randn(8, 8, 3, 3, device=DEV).half(), 128, 0.5),
+                     lambda: layer_norm(fwad.make_dual(x.float(), x.float()), (128,), torch.ones(128, device=DEV), None, 1e-5)):
+            with pytest.raises(RuntimeError, match="forward AD"):
+                call()
