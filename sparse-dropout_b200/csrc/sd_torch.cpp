@@ -13,6 +13,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_cpp_function.h>
@@ -238,7 +239,7 @@ struct PyCallback {
     void operator()() const {
         py::gil_scoped_acquire gil;
         PyObject* r = PyObject_CallNoArgs(f);
-        if (!r) throw py::error_already_set();
+        if (!r) throw_python();
         Py_DECREF(r);
     }
 };
@@ -269,9 +270,11 @@ struct SparseDropLinearBackward : public Node {
         y.reset_data();
     }
     variable_list apply(variable_list&& grads) override;
+    variable_list gradients(variable_list&& grads);
 };
 
-variable_list SparseDropLinearBackward::apply(variable_list&& grads) {
+variable_list SparseDropLinearBackward::apply(variable_list&& grads) { return backward_call([&] { return gradients(std::move(grads)); }); }
+variable_list SparseDropLinearBackward::gradients(variable_list&& grads) {
     at::NoGradGuard no_grad;
     Tensor x16 = x.unpack();
     const Tensor w16 = w.unpack();
@@ -569,7 +572,8 @@ struct SparseDropConv2dBackward : public Node {
         w2d.reset_data();
         cols.reset_data();
     }
-    variable_list apply(variable_list&& grads) override {
+    variable_list apply(variable_list&& grads) override { return backward_call([&] { return gradients(std::move(grads)); }); }
+    variable_list gradients(variable_list&& grads) {
         at::NoGradGuard no_grad;
         const Tensor x16 = x.unpack(), w = w2d.unpack();
         const at::Device dev = x16.device();
@@ -732,7 +736,8 @@ struct SparseDropLayerNormBackward : public Node {
         mean.reset();
         rstd.reset();
     }
-    variable_list apply(variable_list&& grads) override {
+    variable_list apply(variable_list&& grads) override { return backward_call([&] { return gradients(std::move(grads)); }); }
+    variable_list gradients(variable_list&& grads) {
         at::NoGradGuard no_grad;
         const Tensor x2 = x.unpack(), g = weight.unpack();
         const at::Device dev = x2.device();
@@ -865,8 +870,7 @@ PYBIND11_MODULE(sd_torch, m) {
         try {
             if (e) std::rethrow_exception(e);
         } catch (const SdError& err) {
-            static PyObject* type = py::module_::import("flash_dropout._lib").attr("SparseDropError").cast<py::object>().release().ptr();
-            PyErr_SetString(type, err.what());
+            set_python_error(err);
         }
     });
     register_node();

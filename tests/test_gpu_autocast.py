@@ -62,3 +62,16 @@ def test_forward_mode_is_refused(built_lib):
                      lambda: layer_norm(fwad.make_dual(x.float(), x.float()), (128,), torch.ones(128, device=DEV), None, 1e-5)):
             with pytest.raises(RuntimeError, match="forward AD"):
                 call()
+
+
+def test_errors_in_backward_keep_their_type(built_lib):
+    """What the gradient callback raises on autograd's thread is what the caller of backward() catches."""
+    import flash_dropout.functional as F
+    x = torch.randn(128, 128, device=DEV, dtype=torch.float16, requires_grad=True)
+
+    def notify():
+        raise KeyError("bucket")
+
+    y = F.cuda_blockwise_dropout_matmul(x, x.detach(), 128, 0.5, wgrad=(torch.empty(128, 128, device=DEV), False, notify))
+    with pytest.raises(KeyError, match="bucket"):
+        y.sum().backward()
