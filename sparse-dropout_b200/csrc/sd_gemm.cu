@@ -586,6 +586,35 @@ __device__ __forceinline__ void zero_tile(const GemmArgs& g, bool vec_ok, bool v
     }
 }
 
+// Output that no tile of the launch covers is zero-filled by the epilogue warps before their first accumulator is ready: the
+// dropped tiles of an SDD result, the row blocks of a DSD product that keep nothing.  Called by groups of 128 threads; this
+// one takes tile z0 and every zstep-th after it.
+__device__ __forceinline__ void zero_uncovered(const GemmArgs& g, bool vec_ok, bool vec_t_ok, int etid, int lane, int z0, int zstep) {
+    if (g.mode == MODE_SDD && g.n_zero) {
+        const int nz = __ldg(g.n_zero);
+        for (int z = z0; z < nz; z += zstep)
+            zero_tile(g, vec_ok, vec_t_ok, etid, __ldg(g.zero_pairs + 2 * z) * 128, __ldg(g.zero_pairs + 2 * z + 1) * 128);
+    } else if (g.mode == MODE_DSD) {
+        // Every warp of the group tests the same 32 candidates at a time, one per lane, so the index loads of a
+        // whole batch are in flight together; the ballot then gives all of them the same list of tiles to zero.
+        const int ncol = (g.NN + 127) >> 7, total = g.n_row_blocks * ncol;
+        for (int zb = z0; zb < total; zb += 32 * zstep) {
+            const int z = zb + lane * zstep;
+            bool empty = false;
+            if (z < total) {
+                const int rb = z / ncol;
+                empty = __ldg(g.list_ptr + rb + 1) == __ldg(g.list_ptr + rb);
+            }
+            unsigned found = __ballot_sync(0xffffffffu, empty);
+            while (found) {
+                const int zz = zb + (__ffs(found) - 1) * zstep, rb = zz / ncol;
+                found &= found - 1;
+                zero_tile(g, vec_ok, vec_t_ok, etid, rb * 128, (zz - rb * ncol) * 128);
+            }
+        }
+    }
+}
+
 // ------------------------------------------------------------------ epilogue-group helpers
 // Before a warp refills a TMA-store staging buffer: the store that last used it has read it.
 __device__ __forceinline__ void wait_staging_free(bool two_bufs, int n_stores, int lane) {
@@ -1048,32 +1077,7 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
         const bool aligned16 = (reinterpret_cast<uintptr_t>(g.C) & 15) == 0;
         const bool vec_ok = g.c_cs == 1 && (g.c_rs & 7) == 0 && aligned16;      // row-major result, 16-byte rows
         const bool vec_t_ok = g.c_rs == 1 && (g.c_cs & 7) == 0 && aligned16;    // column-major result
-        // Output that no unit covers is zero-filled here, before the first accumulator is ready.
-        if (g.mode == MODE_SDD && g.n_zero) {
-            const int nz = __ldg(g.n_zero);
-            for (int z = epi_halves * cta + half; z < nz; z += epi_halves * n_ctas)
-                zero_tile(g, vec_ok, vec_t_ok, etid, __ldg(g.zero_pairs + 2 * z) * 128, __ldg(g.zero_pairs + 2 * z + 1) * 128);
-        } else if (g.mode == MODE_DSD) {
-            // row blocks with nothing kept: their 128x128 output tiles are spread over all CTAs
-            // Every warp of the group tests the same 32 candidates at a time, one per lane, so the index loads of a
-            // whole batch are in flight together; the ballot then gives all of them the same list of tiles to zero.
-            const int ncol = (g.NN + 127) >> 7, total = g.n_row_blocks * ncol;
-            const int z0 = epi_halves * cta + half, zstep = epi_halves * n_ctas;
-            for (int zb = z0; zb < total; zb += 32 * zstep) {
-                const int z = zb + lane * zstep;
-                bool empty = false;
-                if (z < total) {
-                    const int rb = z / ncol;
-                    empty = __ldg(g.list_ptr + rb + 1) == __ldg(g.list_ptr + rb);
-                }
-                unsigned found = __ballot_sync(0xffffffffu, empty);
-                while (found) {
-                    const int zz = zb + (__ffs(found) - 1) * zstep, rb = zz / ncol;
-                    found &= found - 1;
-                    zero_tile(g, vec_ok, vec_t_ok, etid, rb * 128, (zz - rb * ncol) * 128);
-                }
-            }
-        }
+        zero_uncovered(g, vec_ok, vec_t_ok, etid, lane, epi_halves * cta + half, epi_halves * n_ctas);
         WorkIter it;
         it.init(g, cta, n_ctas, tab);
         int acc = 0;
@@ -1270,6 +1274,12 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
     }
 }
 
+}  // namespace sd
+
+#include "sd_pair.cuh"
+
+namespace sd {
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1288,10 +1298,10 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 // Tensor map of one 16-bit operand X[rows, kk] given its two element strides.
-//   column stride 1 -> K-major : global (kk, rows),  box 64 x 128
+//   column stride 1 -> K-major : global (kk, rows),  box 64 x box_rows
 //   row stride 1    -> MN-major: global (rows, kk),  box 64 x 64
 static int make_operand_map(CUtensorMap* out, bool* mn_major, const char* name, const void* ptr, int64_t rs, int64_t cs,
-                            int rows, int kk, int dtype) {
+                            int rows, int kk, int dtype, int box_rows = 128) {
     if (!ptr) return fail(SD_ERR_INVALID_ARG, "%s is null", name);
     const bool k_major = (cs == 1);
     if (!k_major && rs != 1) return fail(SD_ERR_LAYOUT, "%s must be row or column major", name);
@@ -1313,17 +1323,17 @@ static int make_operand_map(CUtensorMap* out, bool* mn_major, const char* name, 
     }
     // Small per-thread cache: training loops present the same few operands over and over.
     struct MapKey {
-        const void* ptr; int64_t ld; int rows, kk, dtype, dev; bool k_major;
+        const void* ptr; int64_t ld; int rows, kk, dtype, dev, box_rows; bool k_major;
         bool operator==(const MapKey& o) const {
             return ptr == o.ptr && ld == o.ld && rows == o.rows && kk == o.kk && dtype == o.dtype && dev == o.dev &&
-                   k_major == o.k_major;
+                   box_rows == o.box_rows && k_major == o.k_major;
         }
     };
     constexpr int kCache = 32;
     static thread_local MapKey keys[kCache];
     static thread_local CUtensorMap maps[kCache];
     static thread_local int used = 0, next_slot = 0;
-    const MapKey key{ptr, ld, rows, kk, dtype, dev, k_major};
+    const MapKey key{ptr, ld, rows, kk, dtype, dev, box_rows, k_major};
     for (int i = 0; i < used; ++i)
         if (keys[i] == key) {
             *out = maps[i];
@@ -1334,7 +1344,7 @@ static int make_operand_map(CUtensorMap* out, bool* mn_major, const char* name, 
     if (!enc) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable in this driver");
     cuuint64_t dims[2] = {cuuint64_t(inner), cuuint64_t(outer)};
     cuuint64_t strides[1] = {cuuint64_t(outer > 1 ? ld * 2 : ((inner * 2 + 15) & ~int64_t(15)))};
-    cuuint32_t box[2] = {64u, k_major ? 128u : 64u};
+    cuuint32_t box[2] = {64u, k_major ? cuuint32_t(box_rows) : 64u};
     cuuint32_t estr[2] = {1u, 1u};
     CUresult r = enc(out, dtype == SD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                      const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1344,6 +1354,74 @@ static int make_operand_map(CUtensorMap* out, bool* mn_major, const char* name, 
     keys[slot] = key;
     maps[slot] = *out;
     *mn_major = !k_major;
+    return SD_OK;
+}
+
+// Tensor map of a result C[M, N] that leaves by TMA stores (clipped at the ragged edge), and the form in which the epilogue
+// stages it: 16-bit 1 row-major, 2 column-major; fp32 3 column-major, 4 row-major; 0: rows or columns are not 16-byte aligned,
+// the epilogue warps write it themselves.
+static int make_result_map(CUtensorMap* out, int* form, void* C, int M, int N, int64_t c_rs, int64_t c_cs, int dtype, int f32) {
+    const int64_t per16 = f32 ? 4 : 8, size = f32 ? 4 : 2;
+    *form = 0;
+    if (reinterpret_cast<uintptr_t>(C) & 15) return SD_OK;
+    const bool rows = c_cs == 1 && c_rs % per16 == 0 && c_rs >= N, cols = c_rs == 1 && c_cs % per16 == 0 && c_cs >= M;
+    if (!rows && !cols) return SD_OK;
+    const bool row_major = f32 ? !cols : rows;
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable in this driver");
+    const int64_t inner = row_major ? N : M, outer = row_major ? M : N, ld = row_major ? c_rs : c_cs;
+    cuuint64_t dims[2] = {cuuint64_t(inner), cuuint64_t(outer)};
+    cuuint64_t strides[1] = {cuuint64_t(outer > 1 ? ld * size : ((inner * size + 15) & ~int64_t(15)))};
+    cuuint32_t box[2] = {f32 || !row_major ? 32u : 64u, f32 || row_major ? 32u : 64u};
+    cuuint32_t estr[2] = {1u, 1u};
+    const CUtensorMapDataType type = f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                         : dtype == SD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    CUresult r = enc(out, type, 2, C, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     f32 || row_major ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(C) failed with CUresult %d", int(r));
+    *form = f32 ? (row_major ? 4 : 3) : (row_major ? 1 : 2);
+    return SD_OK;
+}
+
+// CTA pairs that can be resident at once on the current device.
+template <bool W_MN, bool S_MN>
+static int pair_capacity(int dev, int* pairs) {
+    static std::atomic<int> known[64] = {};
+    if (dev < 64 && (*pairs = known[dev].load(std::memory_order_relaxed)) > 0) return SD_OK;
+    SD_CUDA_TRY(cudaFuncSetAttribute(sparsedrop_pair_kernel<W_MN, S_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(P_THREADS);
+    cfg.dynamicSmemBytes = P_SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    SD_CUDA_TRY(cudaOccupancyMaxActiveClusters(pairs, sparsedrop_pair_kernel<W_MN, S_MN>, &cfg));
+    if (*pairs <= 0) return fail(SD_ERR_CUDA, "no CTA pair fits this device");
+    if (dev < 64) known[dev].store(*pairs, std::memory_order_relaxed);
+    return SD_OK;
+}
+
+template <bool W_MN, bool S_MN>
+static int launch_pair(const CUtensorMap& tw, const CUtensorMap& ts, const CUtensorMap& tc, const GemmArgs& g, int pairs, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(P_THREADS);
+    cfg.dynamicSmemBytes = P_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    SD_CUDA_TRY(cudaLaunchKernelEx(&cfg, sparsedrop_pair_kernel<W_MN, S_MN>, tw, ts, tc, g));
     return SD_OK;
 }
 
@@ -1409,6 +1487,54 @@ static PlanView view_plan(const void* plan, int R, int C) {
     v.kept_pairs = reinterpret_cast<const int*>(b + L.kept_pairs);
     v.mask = b + L.mask;
     return v;
+}
+
+// The launches that go to the CTA-pair kernel (sd_pair.cuh): a reduction long enough to hide the epilogue of its larger tiles,
+// and work for three quarters of the pairs at 256 columns each.  Either side, single CTAs -> pairs, forward / dX / dW in us:
+//   4096^3 p=0.5 55.8/58.2/57.6 -> 52.2/57.1/52.3, 2500x1352x3016 p=0.3 48.2/46/45.7 -> 42.7/42.2/39.1, 3000^3 p=0.1
+//   64.8/64.3/63 -> 56/58.6/54.9, 16384x4096x4096 p=0.2 306/338/380 -> 297/309-360/358 (limited by power: the tensor pipes
+//   are 86 % busy at 1.5 GHz);
+//   reductions of 384 and 768: 24.2 -> 28.4 (16384x384x1536 dX), 35.7 -> 37.7 (8192x768x3072 dX);
+//   few tiles: 30.3 -> 36.3 (8192x1024x1024 dW, 32 duos), 31.9 -> 65.7 (16384x1536x384 dW, 18 duos), which the split
+//   schedule serves; 50 -> 43 (8192x3072x768 dW, 72 duos).
+static bool pair_serves(const GemmArgs& g, bool special, int sms) {
+    if (special || g.mask_src || g.out_acc || g.KK < 1024) return false;
+    const long long duos = (g.NN + 255) / 256, entries = g.n_row_blocks * ((duos + 1) / 2);
+    if (4 * g.n_row_blocks * duos < 3 * (sms / 2)) return false;
+    if (g.mode == MODE_SDD && g.n_row_blocks > P_MAX_ROW_BLOCKS) return false;
+    return 2 * entries <= (long long)P_TAB_MAX * (sms / 2) && entries <= 16383;      // tables and counters of the kernel
+}
+
+// Launches g on CTA pairs; *taken stays false, with nothing launched, where the result cannot be stored by TMA.
+static int run_pair(GemmArgs g, const void* A, int64_t a_rs, int64_t a_cs, const CUtensorMap& tw, bool w_mn, const void* plan, int dtype,
+                    int sm_margin, cudaStream_t st, bool* taken) {
+    CUtensorMap ts, tc;
+    bool s_mn = false;
+    int rc = make_result_map(&tc, &g.tma_store, g.C, g.NN, g.MM, g.c_cs, g.c_rs, dtype, g.out_f32);   // of the transposed result
+    if (rc || !g.tma_store) return rc;
+    rc = make_operand_map(&ts, &s_mn, "A", A, a_rs, a_cs, g.MM, g.KK, dtype, 64);
+    if (rc) return rc;
+    int dev = 0, pairs = 0;
+    SD_CUDA_TRY(cudaGetDevice(&dev));
+    if (w_mn)
+        rc = s_mn ? pair_capacity<true, true>(dev, &pairs) : pair_capacity<true, false>(dev, &pairs);
+    else
+        rc = s_mn ? pair_capacity<false, true>(dev, &pairs) : pair_capacity<false, false>(dev, &pairs);
+    if (rc) return rc;
+    if (pairs > sm_margin) pairs -= (sm_margin + 1) / 2;
+    g.idesc256 = make_idesc(256, 128, g.is_bf16, w_mn, s_mn);
+    if (g.mode == MODE_SDD) {
+        const PlanView v = view_plan(plan, g.n_row_blocks, (g.NN + 127) / 128);
+        g.list_ptr = v.row_ptr;
+        g.list_idx = v.col_idx;
+    }
+    const long long duos = (g.NN + 255) / 256, most = (long long)g.n_row_blocks * duos;   // duos of the whole result
+    if (most < pairs) pairs = int(most);
+    const long long entries = g.n_row_blocks * ((duos + 1) / 2);
+    if (2 * entries > (long long)P_TAB_MAX * pairs) return SD_OK;   // (halves of the last wave included)
+    *taken = true;
+    if (w_mn) return s_mn ? launch_pair<true, true>(tw, ts, tc, g, pairs, st) : launch_pair<true, false>(tw, ts, tc, g, pairs, st);
+    return s_mn ? launch_pair<false, true>(tw, ts, tc, g, pairs, st) : launch_pair<false, false>(tw, ts, tc, g, pairs, st);
 }
 
 static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const void* B, int64_t b_rs, int64_t b_cs,
@@ -1549,6 +1675,11 @@ static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const v
                         tiles_upper, max_ctas);
         if (grid > max_ctas) grid = max_ctas;
     }
+    if (pair_serves(g, panels != 0 || gather || sdd_t || max_ctas > 0, sms)) {
+        bool taken = false;
+        rc = run_pair(g, A, a_rs, a_cs, tb, b_mn, plan, dtype, sm_margin, static_cast<cudaStream_t>(stream), &taken);
+        if (rc || taken) return rc;
+    }
     // Cutting tiles pays only when each tile is long: the partial-tile exchange costs about as much as a dozen
     // K tiles, so short reductions keep whole tiles even on an under-filled grid.
     const int k_tiles = (K + 127) / 128;
@@ -1588,70 +1719,15 @@ static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const v
     g.tab_min = k_tiles <= 16 ? tab_min_short : TAB_MIN;
     g.use_table = !g.split && (mode != MODE_DSD || k_tiles <= 32) && tiles_upper >= (long long)g.tab_min * grid / 2;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // Row-major result with 16-byte rows: written by TMA (clipped at the ragged edge); otherwise by the warps.
     CUtensorMap tc = ta;
-    if (g.out_f32) {
-        // an fp32 result that overwrites a matrix with 16-byte aligned columns (or rows) leaves by TMA; other
-        // fp32 results (accumulating, unaligned) are written by the epilogue warps directly
-        if (!g.out_acc && c_rs == 1 && (c_cs & 3) == 0 && c_cs >= M && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
-            EncodeTiledFn enc = encode_tiled_fn();
-            cuuint64_t dims[2] = {cuuint64_t(M), cuuint64_t(N)};            // the transpose, row-major [N][M]
-            cuuint64_t strides[1] = {cuuint64_t(N > 1 ? c_cs * 4 : ((int64_t(M) * 4 + 15) & ~int64_t(15)))};
-            cuuint32_t box[2] = {32u, 32u};
-            cuuint32_t estr[2] = {1u, 1u};
-            CUresult r = enc(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(fp32 C^T) failed with CUresult %d", int(r));
-            g.tma_store = 3;
-        } else if (!g.out_acc && c_cs == 1 && (c_rs & 3) == 0 && c_rs >= N && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
-            EncodeTiledFn enc = encode_tiled_fn();
-            cuuint64_t dims[2] = {cuuint64_t(N), cuuint64_t(M)};
-            cuuint64_t strides[1] = {cuuint64_t(M > 1 ? c_rs * 4 : ((int64_t(N) * 4 + 15) & ~int64_t(15)))};
-            cuuint32_t box[2] = {32u, 32u};
-            cuuint32_t estr[2] = {1u, 1u};
-            CUresult r = enc(&tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(fp32 C) failed with CUresult %d", int(r));
-            g.tma_store = 4;
-        }
-    } else if (c_panel_kg) {
-        EncodeTiledFn enc = encode_tiled_fn();
+    if (c_panel_kg) {
         const long long all_rows = (long long)((N + 127) / 128) * c_panel_kg;
         if (all_rows > (1ll << 31) - 1) return fail(SD_ERR_TOO_LARGE, "panel matrix too large");
-        cuuint64_t dims[2] = {128u, cuuint64_t(all_rows)};
-        cuuint64_t strides[1] = {256u};
-        cuuint32_t box[2] = {64u, 32u};
-        cuuint32_t estr[2] = {1u, 1u};
-        CUresult r = enc(&tc, dtype == SD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C,
-                         dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(C panels) failed with CUresult %d", int(r));
-        g.tma_store = 1;
-    } else if (c_cs == 1 && (c_rs & 7) == 0 && c_rs >= N && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
-        EncodeTiledFn enc = encode_tiled_fn();
-        cuuint64_t dims[2] = {cuuint64_t(N), cuuint64_t(M)};
-        cuuint64_t strides[1] = {cuuint64_t(M > 1 ? c_rs * 2 : ((int64_t(N) * 2 + 15) & ~int64_t(15)))};
-        cuuint32_t box[2] = {64u, 32u};
-        cuuint32_t estr[2] = {1u, 1u};
-        CUresult r = enc(&tc, dtype == SD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C,
-                         dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(C) failed with CUresult %d", int(r));
-        g.tma_store = 1;
-    } else if (c_rs == 1 && (c_cs & 7) == 0 && c_cs >= M && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
-        EncodeTiledFn enc = encode_tiled_fn();
-        cuuint64_t dims[2] = {cuuint64_t(M), cuuint64_t(N)};            // the transpose, row-major [N][M]
-        cuuint64_t strides[1] = {cuuint64_t(N > 1 ? c_cs * 2 : ((int64_t(M) * 2 + 15) & ~int64_t(15)))};
-        cuuint32_t box[2] = {32u, 64u};
-        cuuint32_t estr[2] = {1u, 1u};
-        CUresult r = enc(&tc, dtype == SD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, C,
-                         dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(SD_ERR_CUDA, "cuTensorMapEncodeTiled(C^T) failed with CUresult %d", int(r));
-        g.tma_store = 2;
+        rc = make_result_map(&tc, &g.tma_store, C, int(all_rows), 128, 128, 1, dtype, 0);
+    } else if (!g.out_acc) {
+        rc = make_result_map(&tc, &g.tma_store, C, M, N, c_rs, c_cs, dtype, g.out_f32);
     }
+    if (rc) return rc;
     // Epilogue warps (see MAX_EPI_WARPS): four when whole tiles have a long reduction to hide the epilogue behind,
     // eight otherwise.
     static const int epi_warps_env = [] {
