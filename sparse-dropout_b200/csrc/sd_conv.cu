@@ -239,14 +239,14 @@ struct StripGeom {
     int SH, n_strips, CG, n_cgroups;
     int pitch;              // elements per run in shared memory
     int row_lanes;          // lanes that share one image row: a power of two, at most 32
-    int sh_h, sh_w;         // log2 of the strides, or -1
+    int sh_h;               // log2 of the vertical stride, or -1
 };
 __device__ __forceinline__ int div_stride(int v, int stride, int sh, bool* exact) {
     const int q = sh >= 0 ? v >> sh : v / stride;
     *exact = q * stride == v;
     return q;
 }
-template <bool IS_BF16, bool OUT_F32, int SMAX>
+template <bool IS_BF16, bool OUT_F32, int SMAX, int ST>
 __global__ void __launch_bounds__(kConvThreads) col2im_kept_strip_kernel(const unsigned short* __restrict__ dcolT,
                                                                          void* __restrict__ dx, ConvGeom g, StripGeom sg,
                                                                          const unsigned char* __restrict__ tile_mask) {
@@ -262,26 +262,50 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kept_strip_kernel(const u
     const int p0 = max(lo <= 0 ? 0 : (lo + g.stride_h - 1) / g.stride_h, 0), p1 = min(hi / g.stride_h + 1, g.P);
     const int m_first = n * PQ + p0 * g.Q, a0 = m_first & ~7;
     const int nch = p1 > p0 ? (n * PQ + p1 * g.Q - a0 + 7) >> 3 : 0;
-    for (int e = threadIdx.x; e < cn * RS * nch; e += kConvThreads) {
-        const int row = e / nch, ch = e - row * nch;
-        const int k = c0 * RS + row, m = a0 + ch * 8;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (!(tile_mask && __ldg(tile_mask + (long long)(m >> 7) * g.Cb + (k >> 7))))
-            v = __ldg(reinterpret_cast<const uint4*>(dcolT + col_off(g, k, m)));
-        *reinterpret_cast<uint4*>(runs + row * sg.pitch + ch * 8) = v;
+    // four chunks of a thread at a time: their mask bytes, then their loads, are in flight together
+    constexpr int LOADS = 4;
+    for (int e0 = threadIdx.x; e0 < cn * RS * nch; e0 += LOADS * kConvThreads) {
+        int k[LOADS], m[LOADS], at[LOADS];
+        bool on[LOADS];
+        uint4 v[LOADS];
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j) {
+            const int e = e0 + j * kConvThreads, row = e / nch, ch = e - row * nch;
+            at[j] = e < cn * RS * nch ? row * sg.pitch + ch * 8 : -1;
+            k[j] = c0 * RS + row;
+            m[j] = a0 + ch * 8;
+            on[j] = at[j] >= 0 && !(tile_mask && __ldg(tile_mask + (long long)(m[j] >> 7) * g.Cb + (k[j] >> 7)));
+        }
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j) {
+            v[j] = make_uint4(0, 0, 0, 0);
+            if (on[j]) v[j] = __ldg(reinterpret_cast<const uint4*>(dcolT + col_off(g, k[j], m[j])));
+        }
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j)
+            if (at[j] >= 0) *reinterpret_cast<uint4*>(runs + at[j]) = v[j];
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rows_per_warp = 32 / sg.row_lanes, sub = lane / sg.row_lanes, wl = lane - sub * sg.row_lanes;
     const int base0 = n * PQ - a0;                                       // position of output pixel (0, 0) in a run
-    for (int w = wl; w < g.W; w += sg.row_lanes) {
+    // Under a horizontal stride of two (ST == 2) a thread gathers the results w = 2 j and 2 j + 1 of a row: tap s feeds exactly
+    // one of them, the one of the parity of s * dil_w - pad_w, from q = j + const, and every lane has work at every tap.  Under
+    // any other stride (ST == 1) it gathers one, and taps that miss it are skipped.
+    const int J = (g.W + ST - 1) / ST;
+    const bool whole_stores = ST == 2 && !(g.W & 1) && !(reinterpret_cast<uintptr_t>(dx) & 7);
+    unsigned odd = 0;                                                    // ST == 2: taps that feed the second result
+#pragma unroll
+    for (int s = 0; s < SMAX; ++s)
+        if (ST == 2 && ((s * g.dil_w - g.pad_w) & 1)) odd |= 1u << s;
+    for (int j = wl; j < J; j += sg.row_lanes) {
         int q[SMAX];                                                     // where tap s reads in its run, or INT_MIN
 #pragma unroll
         for (int s = 0; s < SMAX; ++s) {
-            const int ww = w + g.pad_w - s * g.dil_w;
-            bool exact;
-            const int qq = div_stride(max(ww, 0), g.stride_w, sg.sh_w, &exact);
-            q[s] = (s < g.S && ww >= 0 && exact && qq < g.Q) ? qq + base0 : INT_MIN;
+            const int ww = ST * j + int(odd >> s & 1) + g.pad_w - s * g.dil_w;
+            const int qq = ST == 2 ? ww >> 1 : g.stride_w == 1 ? ww : max(ww, 0) / g.stride_w;
+            const bool exact = ST == 2 || qq * g.stride_w == ww;
+            q[s] = (s < g.S && ww >= 0 && exact && qq < g.Q) ? s * sg.pitch + qq + base0 : INT_MIN;
         }
         // (channel, input row) pairs of this thread, without a division per pair
         const int rows = h1 - h0, step = (kConvThreads / 32) * rows_per_warp;
@@ -291,33 +315,43 @@ __global__ void __launch_bounds__(kConvThreads) col2im_kept_strip_kernel(const u
             if (cg >= cn) break;
             const unsigned short* src = runs + cg * RS * sg.pitch;
             const int top = h0 + h + g.pad_h;
-            float acc = 0.f;
+            float acc[ST] = {};
+            auto add_row = [&](const unsigned short* at) {
+#pragma unroll
+                for (int s = 0; s < SMAX; ++s)
+                    if (q[s] != INT_MIN) {
+                        const float f = to_float(at[q[s]], IS_BF16);
+                        if (ST == 2 && (odd >> s & 1)) acc[ST - 1] += f; else acc[0] += f;
+                    }
+            };
             if (g.dil_h == 1) {
                 // the filter rows that meet an output row: every stride_h-th one
                 int r = sg.sh_h == 0 ? 0 : sg.sh_h > 0 ? top & (g.stride_h - 1) : top % g.stride_h;
                 int p = sg.sh_h >= 0 ? (top - r) >> sg.sh_h : (top - r) / g.stride_h;
                 if (p >= g.P) { r += (p - g.P + 1) * g.stride_h; p = g.P - 1; }
-                for (; r < g.R && p >= 0; r += g.stride_h, --p) {
-                    const unsigned short* at = src + r * g.S * sg.pitch + p * g.Q;
-#pragma unroll
-                    for (int s = 0; s < SMAX; ++s)
-                        if (q[s] != INT_MIN) acc += to_float(at[s * sg.pitch + q[s]], IS_BF16);
-                }
+                for (; r < g.R && p >= 0; r += g.stride_h, --p) add_row(src + r * g.S * sg.pitch + p * g.Q);
             } else {
                 for (int r = 0; r < g.R; ++r) {
                     const int hh = top - r * g.dil_h;
                     bool exact;
                     const int p = div_stride(max(hh, 0), g.stride_h, sg.sh_h, &exact);
                     if (hh < 0 || !exact || p >= g.P) continue;
-                    const unsigned short* at = src + r * g.S * sg.pitch + p * g.Q;
-#pragma unroll
-                    for (int s = 0; s < SMAX; ++s)
-                        if (q[s] != INT_MIN) acc += to_float(at[s * sg.pitch + q[s]], IS_BF16);
+                    add_row(src + r * g.S * sg.pitch + p * g.Q);
                 }
             }
-            const long long i = ((long long)(n * g.C + c0 + cg) * g.H + h0 + h) * g.W + w;
-            if (OUT_F32) static_cast<float*>(dx)[i] = acc;
-            else static_cast<unsigned short*>(dx)[i] = from_float(acc, IS_BF16);
+            const long long i = ((long long)(n * g.C + c0 + cg) * g.H + h0 + h) * g.W + ST * j;
+            if (whole_stores) {                                          // both results in one store
+                if (OUT_F32) *reinterpret_cast<float2*>(static_cast<float*>(dx) + i) = make_float2(acc[0], acc[ST - 1]);
+                else *reinterpret_cast<uint32_t*>(static_cast<unsigned short*>(dx) + i) =
+                         from_float(acc[0], IS_BF16) | (uint32_t(from_float(acc[ST - 1], IS_BF16)) << 16);
+            } else {
+#pragma unroll
+                for (int b = 0; b < ST; ++b)
+                    if (ST * j + b < g.W) {
+                        if (OUT_F32) static_cast<float*>(dx)[i + b] = acc[b];
+                        else static_cast<unsigned short*>(dx)[i + b] = from_float(acc[b], IS_BF16);
+                    }
+            }
         }
     }
 }
@@ -598,10 +632,9 @@ static bool strip_geom(const ConvGeom& g, uintptr_t src, StripGeom* sg, int* byt
     sg->n_cgroups = (g.C + CG - 1) / CG;
     sg->pitch = int(run_elems(SH));
     sg->row_lanes = 1;
-    while (sg->row_lanes < g.W && sg->row_lanes < 32) sg->row_lanes *= 2;
+    while (sg->row_lanes * (g.stride_w == 2 ? 2 : 1) < g.W && sg->row_lanes < 32) sg->row_lanes *= 2;
     auto log2_or = [](int v) { int l = 0; while ((1 << l) < v) ++l; return (1 << l) == v ? l : -1; };
     sg->sh_h = log2_or(g.stride_h);
-    sg->sh_w = log2_or(g.stride_w);
     if ((long long)g.N * sg->n_cgroups * sg->n_strips > (1ll << 31) - 1) return false;
     *bytes = int(one * CG);
     return true;
@@ -684,8 +717,9 @@ static int col2im_kept_impl(const void* dcolT, int64_t ldm, int k_gemm, int N, i
     else if (sd::strip_geom(g, reinterpret_cast<uintptr_t>(dcolT), &sg, &strip_bytes)) {
         const unsigned n_cta = unsigned(N) * sg.n_cgroups * sg.n_strips;
         by_type([&](auto bf, auto f32) {
-            if (S <= 3) sd::col2im_kept_strip_kernel<bf.value, f32.value, 3><<<n_cta, sd::kConvThreads, strip_bytes, st>>>(src, dx, g, sg, mask);
-            else sd::col2im_kept_strip_kernel<bf.value, f32.value, 7><<<n_cta, sd::kConvThreads, strip_bytes, st>>>(src, dx, g, sg, mask);
+            auto kernel = S <= 3 ? (stride_w != 2 ? &sd::col2im_kept_strip_kernel<bf.value, f32.value, 3, 1> : &sd::col2im_kept_strip_kernel<bf.value, f32.value, 3, 2>)
+                                 : (stride_w != 2 ? &sd::col2im_kept_strip_kernel<bf.value, f32.value, 7, 1> : &sd::col2im_kept_strip_kernel<bf.value, f32.value, 7, 2>);
+            kernel<<<n_cta, sd::kConvThreads, strip_bytes, st>>>(src, dx, g, sg, mask);
         });
     } else
         sd::col2im_kept_kernel<<<grid, sd::kConvThreads, 0, st>>>(src, dx, g, mask, dtype == SD_BF16, out_f32);

@@ -12,6 +12,8 @@ GEOMS = [  # N, C, H, W, R, S, padding, stride, dilation
     (2, 4, 33, 30, 3, 3, (1, 1), (2, 2), (1, 1)),     # strides that are a power of two, odd height
     (1, 4, 20, 23, 3, 2, (2, 0), (3, 3), (1, 1)),     # strides that are not, input rows no output row reads
     (2, 3, 17, 19, 3, 3, (2, 2), (1, 2), (2, 2)),     # dilated rows and columns
+    (2, 3, 18, 21, 3, 3, (1, 1), (2, 2), (1, 1)),     # pairs of results with an odd width: the last pair is cut, single stores
+    (1, 3, 56, 70, 5, 5, (2, 2), (2, 2), (1, 1)),     # more pairs than lanes; taps of either parity
     (1, 2, 14, 15, 1, 7, (0, 3), (1, 1), (1, 1)),     # the widest filter the strips take
     (1, 2, 14, 15, 2, 9, (0, 4), (2, 1), (1, 1)),     # one wider: element by element
     (2, 4, 16, 16, 3, 3, (1, 1), (1, 1), (1, 1)),     # the 3x3 kernel with an fp32 result
