@@ -395,6 +395,14 @@ int sd_layernorm_bwd(const float* x, const void* dy, int dy_dtype, const float* 
                      void* workspace, void* stream);
 
 /* ------------------------------------------------------------------------------------------
+ * GELU (x * Phi(x), the exact form) between the two SparseDrop layers of a transformer MLP (eval/llm/model.py:60-69), on
+ * contiguous 16-byte aligned tensors of n elements of SD_F16 or SD_BF16, computed in fp32 and rounded once:
+ *   forward : y = x * Phi(x);   backward: dx = dy * (Phi(x) + x * phi(x))
+ * ------------------------------------------------------------------------------------------ */
+int sd_gelu_fwd(const void* x, void* y, int64_t n, int dtype, void* stream);
+int sd_gelu_bwd(const void* dy, const void* x, void* dx, int64_t n, int dtype, void* stream);
+
+/* ------------------------------------------------------------------------------------------
  * AdamW over all parameters of a model in one launch (the reference trains with torch.optim.AdamW(fused=True),
  * eval/llm/model.py:157-173).  Every tensor is contiguous fp32 in device memory, 16-byte aligned; `step` is its step counter
  * (one float, as torch keeps it), which the launch advances by one.  Per element, with t the advanced counter:

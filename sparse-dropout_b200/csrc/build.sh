@@ -17,7 +17,7 @@ torch_job=$!
     -Xcompiler -fPIC -Xptxas -v --shared \
     -o "$out/libsparsedrop.so" \
     "$here/sd_api.cu" "$here/sd_plan.cu" "$here/sd_gemm.cu" "$here/sd_conv.cu" "$here/sd_norm.cu" "$here/sd_cast.cu" \
-    "$here/sd_optim.cu" "$here/sd_selftest.cu" "$@"
+    "$here/sd_optim.cu" "$here/sd_gelu.cu" "$here/sd_selftest.cu" "$@"
 wait $torch_job
 "${CXX:-g++}" -shared -o "$out/sd_torch.so" "$out/sd_torch.o" -L"$out" -lsparsedrop -L"$torch/lib" -lc10 -lc10_cuda -ltorch_cpu \
     -ltorch_cuda -ltorch_python -Wl,-rpath,'$ORIGIN' -Wl,-rpath,"$torch/lib"

@@ -9,6 +9,7 @@
 // Replaces the glue of flash_dropout/functional/blockwise_dropout_matmul_cuda.py:7-59 and
 // flash_dropout/cuda/src/gemm_binding.cu:44-141.
 #include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -806,6 +807,52 @@ std::optional<Tensor> layer_norm(const Tensor& x, const Tensor& weight, const st
     return y;
 }
 
+// ---------------------------------------------------------------- GELU
+inline bool aligned16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
+struct SparseDropGeluBackward : public Node {
+    SavedVariable x;
+
+    std::string name() const override { return "SparseDropGeluBackward"; }
+    void release_variables() override { x.reset_data(); }
+    variable_list apply(variable_list&& grads) override { return backward_call([&] { return gradients(std::move(grads)); }); }
+    variable_list gradients(variable_list&& grads) {
+        if (!grads[0].defined()) return {Tensor()};
+        const Tensor h = x.unpack();
+        if (at::GradMode::is_enabled()) return {at::gelu_backward(grads[0], h)};     // the gradient's own graph is wanted
+        Tensor dy = grads[0];
+        if (dy.scalar_type() != h.scalar_type()) dy = dy.to(h.scalar_type());
+        dy = dy.contiguous();
+        if (!aligned16(dy)) dy = dy.clone();
+        const Tensor hc = h.is_contiguous() && aligned16(h) ? h : h.clone(at::MemoryFormat::Contiguous);   // (a hook may unpack another layout)
+        const at::Device dev = hc.device();
+        c10::cuda::OptionalCUDAGuard guard(dev);
+        Tensor dx = at::detail::empty_cuda(hc.sizes(), hc.scalar_type(), dev, std::nullopt);
+        check_rc(sd_gelu_bwd(dy.data_ptr(), hc.data_ptr(), dx.data_ptr(), hc.numel(), dtype_code(hc.scalar_type()),
+                             c10::cuda::getCurrentCUDAStream(dev.index()).stream()));
+        return {dx};
+    }
+};
+
+// Nothing if the kernels do not serve this tensor: a plain contiguous 16-bit one on a CUDA device.
+std::optional<Tensor> gelu(const Tensor& x) {
+    py::gil_scoped_release no_gil;
+    const at::ScalarType t = x.scalar_type();
+    if (!x.is_cuda() || (t != at::kHalf && t != at::kBFloat16) || at::isTensorSubclassLike(x) || !x.is_contiguous() || !x.numel() ||
+        !aligned16(x) || torch::autograd::isFwGradDefined(x))
+        return std::nullopt;
+    const at::Device dev = x.device();
+    c10::cuda::OptionalCUDAGuard guard(dev);
+    Tensor y = at::detail::empty_cuda(x.sizes(), t, dev, std::nullopt);
+    check_rc(sd_gelu_fwd(x.data_ptr(), y.data_ptr(), x.numel(), dtype_code(t), c10::cuda::getCurrentCUDAStream(dev.index()).stream()));
+    if (!torch::autograd::compute_requires_grad(x)) return y;
+    std::shared_ptr<SparseDropGeluBackward> node(new SparseDropGeluBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x));
+    node->x = SavedVariable(x, false);
+    torch::autograd::set_history(y, node);
+    return y;
+}
+
 // ---------------------------------------------------------------- AdamW
 // The tensors of one optimizer, described to the kernel once; a step checks that none of them has moved since.  Only weak
 // references are held: parameters lead back to whoever holds this object (their gradient hooks), and Python's collector
@@ -880,6 +927,7 @@ PYBIND11_MODULE(sd_torch, m) {
     m.def("gemm_dsd", &gemm_dsd);
     m.def("gemm_sdd", &gemm_sdd);
     m.def("layer_norm", &layer_norm);
+    m.def("gelu", &gelu);
     py::class_<AdamW>(m, "AdamW")
         .def(py::init<const std::vector<std::array<Tensor, 5>>&, const std::vector<int64_t>&>())
         .def("step", &AdamW::step);

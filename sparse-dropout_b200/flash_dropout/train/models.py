@@ -15,6 +15,7 @@ import torch.nn.functional as F
 from torch import nn
 
 from flash_dropout.layers import DropoutMM
+from flash_dropout.layers.gelu import GELU
 from flash_dropout.layers.norm import LayerNorm
 
 
@@ -68,7 +69,7 @@ class MLP(nn.Module):
     def __init__(self, n_embed: int, dropout: dict):
         super().__init__()
         self.c_fc = DropoutMM(n_embed, 4 * n_embed, **dropout)
-        self.gelu = nn.GELU()
+        self.gelu = GELU()
         self.c_proj = DropoutMM(4 * n_embed, n_embed, **dropout)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
@@ -165,7 +166,7 @@ class ViTTransformer(nn.Module):
         self.layers = nn.ModuleList(
             nn.ModuleList([
                 ViTSelfAttention(n_embed, n_head, dropout),
-                nn.Sequential(LayerNorm(n_embed), DropoutMM(n_embed, 4 * n_embed, **dropout), nn.GELU(),
+                nn.Sequential(LayerNorm(n_embed), DropoutMM(n_embed, 4 * n_embed, **dropout), GELU(),
                               DropoutMM(4 * n_embed, n_embed, **dropout)),
             ]) for _ in range(n_layers))
 
