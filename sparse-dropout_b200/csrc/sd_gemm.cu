@@ -67,11 +67,15 @@ constexpr int TILE_SMEM = STAGES * STAGE_BYTES;          // 192 KiB
 // warps only take issue slots from the producer and MMA warps.
 constexpr int MAX_EPI_WARPS = 8;
 constexpr int STAGING_BYTES = 8 * 4096;                  // TMA-store staging
-// Tile table: a CTA that runs several whole-tile passes resolves all of them once, in its prologue, into shared
-// memory (row block, column tile, keep bits of the row block's K tiles), so that no role pays the chain of
-// dependent index loads (order -> list bounds -> list entries) again for every tile.
-constexpr int TAB_MAX = 96, TAB_MIN = 8;
+// Tile table: a CTA that runs several whole-tile passes resolves all of them once, in its prologue, into shared memory (row
+// block, column tile, keep bits of the row block's K tiles), so that no role walks the plan's indexes again for every tile.  For
+// a DSD product a warp takes a pass: its lanes read the row block's mask bytes together, one round trip.
+constexpr int TAB_MAX = 96;
 constexpr int TAB_BYTES = TAB_MAX * 16;
+// The split schedule's prologue keeps the first CTA of every tile's group and this CTA's own part in the same place.
+constexpr int SPLIT_MAX_TILES = 256;
+struct SplitSeg { int tile, owner, parts, part, beg, nk; };   // parts == 0: nothing for this CTA
+static_assert(SPLIT_MAX_TILES * 4 + sizeof(SplitSeg) <= TAB_BYTES, "shares the table's memory");
 constexpr int GEMM_SMEM = TILE_SMEM + 1024 /*align*/ + 256 /*barriers*/ + STAGING_BYTES + TAB_BYTES;
 static_assert(GEMM_SMEM <= 227 * 1024, "over the shared memory of one CTA");
 constexpr int GEMM_MAX_THREADS = 96 + MAX_EPI_WARPS * 32;   // producer A, MMA, epilogue warps, producer B
@@ -155,12 +159,11 @@ struct GemmArgs {
                                      // major; fp32 3 column-major, 4 row-major
     float* ws_slots;
     int* ws_flags;
-    const unsigned char* direct_mask;   // DSD launches in which a CTA gets only a few tiles: the plan's tile mask
-    int dm_stride_rb, dm_stride_k;      // (1 = dropped), byte (row block rb, K tile k) at rb * dm_stride_rb + k * dm_stride_k.
-                                        // A CTA then reads its row block's <= 32 mask bytes in one round trip instead of
-                                        // walking order -> list bounds -> list entries (three dependent loads)
+    const unsigned char* direct_mask;   // DSD with at most 32 K tiles: the plan's tile mask (1 = dropped), byte (row block
+    int dm_stride_rb, dm_stride_k;      // rb, K tile k) at rb * dm_stride_rb + k * dm_stride_k
     int use_table;                   // whole-tile schedule whose tiles can be described by the shared-memory table
     int tab_min;                     // fewest passes of a CTA from which the table is used
+    int bn;                          // split schedule: width of a column tile, 256 or 128
     int all_halves;                  // whole-tile schedule of a launch that would leave most SMs idle: every tile is
                                      // handed out as two 128-wide halves, so twice as many SMs stream the operands
     int act;                         // epilogue: 1 = ReLU on the result (eval/mlp/model.py:33-38 applies it as a separate op)
@@ -221,16 +224,19 @@ struct KIter {
 //   split == 1 : every output tile gets a group of consecutive CTAs, sized in proportion to the tile's
 //                work, and each CTA of the group one contiguous part of the tile's kept K-tile list (see
 //                the file header); the choice when there are fewer tiles than SMs and a long reduction.
+// The schedule is a compile-time choice: a launch is bound by fetching cold instructions as much as by anything else when it is
+// small, and code of the other schedule between the roles cost one at 512^3 0.45 us.
+template <bool SPLIT>
 struct WorkIter {
     int t, n_tiles, stride, pass;   // whole tiles: this CTA's index, tile count, gridDim.x, next pass
     int nk_uniform;              // dense / SDD: K tiles per output tile
     int full_per_row, n_full;    // whole tiles: full-width column tiles per row block, and in total
     int whole_entries, n_entries;   // whole tiles: list entries that are whole tiles, and all entries (see init)
-    int sp_rb, sp_nt, sp_owner, sp_parts, sp_part;   // split: this CTA's one segment; sp_parts == 0: none
-    bool split, snake;
+    SplitSeg sp;                 // split: this CTA's one segment
+    bool snake;
     const int4* tab;             // shared-memory tile table (see TAB_MAX), or null: resolve every tile from the plan
     int passes;                  // whole tiles: passes over the entry list this grid makes
-    bool direct;                 // DSD, few passes: tiles resolved from the plan's mask bytes (see GemmArgs::direct_mask)
+    bool direct;                 // DSD, one pass: the tile is resolved from the plan's mask bytes (see GemmArgs::direct_mask)
 
     __device__ __forceinline__ int count(const GemmArgs& g, int r) const {
         return __ldg(g.list_ptr + r + 1) - __ldg(g.list_ptr + r);
@@ -253,10 +259,15 @@ struct WorkIter {
                                       : unsigned((unsigned long long)spare * w / total);
         return tile + int(extra);
     }
+    // `table`: the CTA's tile table, or where split_prologue left its part.
     __device__ void init(const GemmArgs& g, int cta, int n_ctas, const int4* table) {
-        split = g.split != 0;
         tab = nullptr;
         nk_uniform = (g.KK + 127) >> 7;
+        pass = 0;
+        if (SPLIT) {
+            sp = *reinterpret_cast<const SplitSeg*>(reinterpret_cast<const int*>(table) + SPLIT_MAX_TILES);
+            return;
+        }
         if (g.mode == MODE_SDD && g.sdd_single == 3) {
             n_tiles = 0;
             for (int c = 0; c < g.n_row_blocks; ++c) n_tiles += (count(g, c) + 1) >> 1;
@@ -265,13 +276,9 @@ struct WorkIter {
         }
         t = cta;
         stride = n_ctas;
-        pass = 0;
         // with equal tiles (dense, SDD, a mask that dropped nothing) plain round-robin keeps neighbouring CTAs on
         // neighbouring tiles in every pass; see below for unequal row blocks
-        direct = false;
         snake = false;
-        sp_rb = sp_nt = sp_owner = sp_part = 0;
-        sp_parts = 0;
         const bool ragged = (g.n_col_tiles - 1) * BN + 128 >= g.NN;
         full_per_row = (ragged && g.n_col_tiles > 1) ? g.n_col_tiles - 1 : g.n_col_tiles;
         n_full = g.n_row_blocks * full_per_row;
@@ -288,33 +295,42 @@ struct WorkIter {
         }
         n_entries = whole_entries + 2 * (n_tiles - whole_entries);
         passes = (n_entries + n_ctas - 1) / n_ctas;
-        direct = g.direct_mask != nullptr && !split && passes < g.tab_min;
         // alternate the direction only when row blocks differ in length (and there is more than one pass)
         if (g.mode == MODE_DSD && passes > 1) snake = __ldg(g.h_nnz) != g.n_row_blocks * __ldg(g.h_max);
-        // the table costs a CTA-wide barrier and one chain of index loads up front: worth it from a handful of tiles per
-        // CTA on (the short tiles of a conv), not for the three or four long tiles of a large square product
-        if (g.use_table && !split && passes >= g.tab_min && passes <= TAB_MAX) tab = table;
-        if (!split || n_tiles == 0 || n_tiles > n_ctas) return;
+        if (g.use_table && passes >= g.tab_min && passes <= TAB_MAX) tab = table;
+        direct = g.direct_mask != nullptr && !tab;
+    }
+    // Prologue of a CTA under the split schedule: all threads together find the tile whose group this CTA belongs to.  The
+    // list bounds of all tiles are read in one round trip (a search by each role took ~7000 cycles at 9 tiles).
+    __device__ void split_prologue(const GemmArgs& g, int cta, int n_ctas, void* table, int tid, int n_threads) {
+        int* start = static_cast<int*>(table);
+        SplitSeg* out = reinterpret_cast<SplitSeg*>(start + SPLIT_MAX_TILES);
+        nk_uniform = (g.KK + 127) >> 7;
+        n_tiles = g.mode == MODE_SDD ? __ldg(g.n_items) : g.n_row_blocks * g.n_col_tiles;
+        const bool ragged = g.bn == BN && (g.n_col_tiles - 1) * BN + 128 >= g.NN;
         const int row_weight = 2 * g.n_col_tiles - (ragged ? 1 : 0);
-        const unsigned total = work_before(g, n_tiles, row_weight);
-        if (total == 0) return;                                   // everything dropped: only zero-filling is left
+        const unsigned total = (n_tiles > 0 && n_tiles <= n_ctas) ? work_before(g, n_tiles, row_weight) : 0;
         const int spare = n_ctas - n_tiles;
         const bool fits32 = (unsigned long long)total * unsigned(spare) <= 0xffffffffull;
-        int lo = 0, hi = n_tiles - 1;                             // last tile whose group starts at or before this CTA
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (group_start(g, mid, row_weight, total, spare, fits32) <= cta) lo = mid; else hi = mid - 1;
-        }
-        const int first = group_start(g, lo, row_weight, total, spare, fits32);
-        const int next_first = lo + 1 < n_tiles ? group_start(g, lo + 1, row_weight, total, spare, fits32) : n_ctas;
-        if (g.mode == MODE_SDD) { sp_rb = lo; sp_nt = 0; }
-        else { sp_rb = lo / g.n_col_tiles; sp_nt = lo - sp_rb * g.n_col_tiles; }
-        const int nk = g.mode == MODE_DSD ? count(g, sp_rb) : nk_uniform;
-        int parts = next_first - first;
-        if (parts > nk) parts = nk;                               // never more CTAs on a tile than it has K tiles
-        sp_owner = first;
-        sp_part = cta - first;
-        sp_parts = sp_part < parts ? parts : 0;
+        if (tid == 0) out->parts = 0;             // everything dropped: only zero-filling is left
+        if (total)
+            for (int t = tid; t < n_tiles; t += n_threads) start[t] = group_start(g, t, row_weight, total, spare, fits32);
+        __syncthreads();
+        if (total)
+            for (int t = tid; t < n_tiles; t += n_threads) {
+                const int first = start[t], end = t + 1 < n_tiles ? start[t + 1] : n_ctas;
+                if (cta < first || cta >= end) continue;          // groups do not overlap: one thread goes on
+                SplitSeg o{t, first, 0, cta - first, 0, nk_uniform};
+                if (g.mode == MODE_DSD) {
+                    const int rb = t / g.n_col_tiles;
+                    o.beg = __ldg(g.list_ptr + rb);
+                    o.nk = __ldg(g.list_ptr + rb + 1) - o.beg;
+                }
+                const int parts = min(end - first, o.nk);         // never more CTAs on a tile than it has K tiles
+                o.parts = o.part < parts ? parts : 0;
+                *out = o;
+            }
+        __syncthreads();
     }
     __device__ __forceinline__ void fill(const GemmArgs& g, Seg& s, int row_block, int n_tile) const {
         s.bits = 0;
@@ -366,23 +382,41 @@ struct WorkIter {
     // for this CTA.  Pass j hands out entries [j*stride, (j+1)*stride) of the heaviest-first list; with unequal row
     // blocks, forwards on even passes and backwards on odd ones, so the CTA that got the heaviest tile of one pass gets
     // the lightest of the next.
-    __device__ bool resolve(const GemmArgs& g, int ps, Seg& s) const {
+    // locate: the tile, and its half or -1; resolve: everything else, from the plan's lists.
+    __device__ bool locate(int ps, int& tile, int& half) const {
         const int entry = ps * stride + (((ps & 1) && snake) ? stride - 1 - t : t);   // pass 0 does not wait for `snake`
         if (entry >= n_entries) return false;
-        const int tile = entry < whole_entries ? entry : whole_entries + ((entry - whole_entries) >> 1);
-        const int half = entry < whole_entries ? -1 : ((entry - whole_entries) & 1);
+        tile = entry < whole_entries ? entry : whole_entries + ((entry - whole_entries) >> 1);
+        half = entry < whole_entries ? -1 : ((entry - whole_entries) & 1);
+        return true;
+    }
+    // Row block (as a place in the heaviest-first order) and column tile.  List order: row blocks heaviest first, and when the
+    // last column tile is only 128 wide (half the work), all full-width tiles before all narrow ones, so that no CTA
+    // collects only full-width tiles.
+    __device__ void place(const GemmArgs& g, int tile, int& rbi, int& nt) const {
+        if (tile < n_full) { rbi = tile / full_per_row; nt = tile - rbi * full_per_row; }
+        else { rbi = tile - n_full; nt = g.n_col_tiles - 1; }
+    }
+    // One 128-wide half of a tile of the last wave; false if the tile is only 128 wide and this would be its second half.
+    static __device__ bool cut(int half, int& b_row0, int& b_row1) {
+        if (half < 0) return true;
+        if (b_row1 < 0) return half == 0;
+        if (half == 1) b_row0 = b_row1;
+        b_row1 = -1;
+        return true;
+    }
+    __device__ bool resolve(const GemmArgs& g, int ps, Seg& s) const {
+        int tile, half;
+        if (!locate(ps, tile, half)) return false;
         if (g.mode == MODE_SDD) {
             fill(g, s, tile, 0);
         } else {
-            // list order: row blocks heaviest first, and when the last column tile is only 128 wide (half the
-            // work), all full-width tiles before all narrow ones, so that no CTA collects only full-width tiles
             int rbi, nt;
-            if (tile < n_full) { rbi = tile / full_per_row; nt = tile - rbi * full_per_row; }
-            else { rbi = tile - n_full; nt = g.n_col_tiles - 1; }
+            place(g, tile, rbi, nt);
+            const int rb = passes > 1 && g.order ? __ldg(g.order + rbi) : rbi;   // with one pass the order does not matter
             if (direct) {
-                // the kept K tiles come straight from the mask bytes of the row block (with one pass the order of the
-                // tiles does not matter either)
-                const int rb = (passes > 1 && g.order) ? __ldg(g.order + rbi) : rbi;
+                // the kept K tiles come straight from the mask bytes of the row block (each role for itself: handing one
+                // warp's ballot to the others through the table cost a launch at 512^3 0.25 us more)
                 const unsigned char* m = g.direct_mask + (long long)rb * g.dm_stride_rb;
                 uint32_t bits = 0;
                 for (int j = 0; j < nk_uniform; ++j) bits |= uint32_t(__ldg(m + (long long)j * g.dm_stride_k) == 0) << j;
@@ -394,39 +428,45 @@ struct WorkIter {
                 s.bits = bits;
                 s.nk = __popc(bits);
             } else {
-                fill(g, s, g.order ? __ldg(g.order + rbi) : rbi, nt);
+                fill(g, s, rb, nt);
             }
         }
         if (s.nk == 0) return false;          // empty row blocks are zero-filled by the epilogue warps
-        if (half >= 0) {                      // one 128-wide half of a tile of the last wave
-            if (s.b_row1 < 0) {
-                if (half == 1) return false;  // the tile is only 128 wide: there is no second half
-            } else {
-                if (half == 1) s.b_row0 = s.b_row1;
-                s.b_row1 = -1;
-            }
-        }
+        if (!cut(half, s.b_row0, s.b_row1)) return false;
         s.i0 = 0;
         s.i1 = s.nk;
         s.owner = 0; s.parts = 1; s.part = 0;
         return true;
     }
-    // Prologue of a CTA that uses the tile table: every thread resolves some of the passes.
+    // Prologue of a CTA that uses the tile table.
     __device__ void fill_table(const GemmArgs& g, int4* table, int tid, int n_threads) const {
+        if (g.mode == MODE_DSD) {
+            const int lane = tid & 31;
+            for (int ps = tid >> 5; ps < passes; ps += n_threads >> 5) {
+                int tile, half;
+                int4 e = make_int4(-1, 0, 0, 0);
+                if (locate(ps, tile, half)) {
+                    int rbi, nt;
+                    place(g, tile, rbi, nt);
+                    const int rb = passes > 1 && g.order ? __ldg(g.order + rbi) : rbi;
+                    const unsigned char* m = g.direct_mask + (long long)rb * g.dm_stride_rb;
+                    const uint32_t bits = __ballot_sync(0xffffffffu, lane < nk_uniform && __ldg(m + (long long)lane * g.dm_stride_k) == 0);
+                    int b0 = nt * BN, b1 = (nt * BN + 128 < g.NN) ? nt * BN + 128 : -1;
+                    if (bits && cut(half, b0, b1)) e = make_int4(rb * 128, b0, b1, int(bits));
+                }
+                if (lane == 0) table[ps] = e;
+            }
+            return;
+        }
         for (int ps = tid; ps < passes; ps += n_threads) {
             Seg s;
             int4 e = make_int4(-1, 0, 0, 0);
-            if (resolve(g, ps, s)) {
-                uint32_t bits = 0;
-                if (g.mode == MODE_DSD)
-                    for (int j = 0; j < s.nk; ++j) bits |= 1u << __ldg(s.klist + j);
-                e = make_int4(s.a_row, s.b_row0, s.b_row1, int(bits));
-            }
+            if (resolve(g, ps, s)) e = make_int4(s.a_row, s.b_row0, s.b_row1, 0);
             table[ps] = e;
         }
     }
     __device__ bool next(const GemmArgs& g, Seg& s) {
-        if (!split) {
+        if (!SPLIT) {
             if (tab) {
                 for (; pass < passes; ++pass) {
                     const int4 e = tab[pass];
@@ -451,12 +491,23 @@ struct WorkIter {
             }
             return false;
         }
-        if (sp_parts == 0) return false;
-        fill(g, s, sp_rb, sp_nt);
-        s.i0 = s.nk * sp_part / sp_parts;
-        s.i1 = s.nk * (sp_part + 1) / sp_parts;
-        s.owner = sp_owner; s.parts = sp_parts; s.part = sp_part;
-        sp_parts = 0;                             // one segment per CTA
+        if (sp.parts == 0) return false;
+        if (g.mode == MODE_SDD) {
+            fill(g, s, sp.tile, 0);
+        } else {
+            const int rb = sp.tile / g.n_col_tiles, col = (sp.tile - rb * g.n_col_tiles) * g.bn;
+            s.a_row = rb * 128;
+            s.b_row0 = col;
+            s.b_row1 = g.bn == BN && col + 128 < g.NN ? col + 128 : -1;
+            s.klist = g.mode == MODE_DSD ? g.list_idx + sp.beg : nullptr;
+            s.nk = sp.nk;
+            s.bits = 0;
+            s.use_bits = false;
+        }
+        s.i0 = int((long long)s.nk * sp.part / sp.parts);
+        s.i1 = int((long long)s.nk * (sp.part + 1) / sp.parts);
+        s.owner = sp.owner; s.parts = sp.parts; s.part = sp.part;
+        sp.parts = 0;                             // one segment per CTA
         return true;
     }
 };
@@ -680,8 +731,8 @@ __device__ bool reduce_shared_tile(const GemmArgs& g, const Seg& seg, int eidx, 
     const int n_units = (seg.b_row1 >= 0 ? 8 : 4) * 4;
     unsigned short* C = static_cast<unsigned short*>(g.C);
     const bool quad_ok = g.c_cs == 1 && (g.c_rs & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 7) == 0;
-    // A unit is 8 four-column pieces x 32 rows of 16 bytes, shared by all epilogue threads.  The loads of four partial
-    // tiles are kept in flight at once, so the depth of the dependent chain is P / 4 round trips.
+    // A unit is 8 four-column pieces x 32 rows of 16 bytes, shared by all epilogue threads.  The loads of eight partial
+    // tiles are kept in flight at once, so the depth of the dependent chain is P / 8 round trips.
     for (int uu = my_index; uu < n_units; uu += P) {
       const int c = uu >> 2, q = uu & 3;
       for (int e = eidx; e < 256; e += epi_threads) {            // piece index inside the unit: [4-column piece][row]
@@ -689,17 +740,16 @@ __device__ bool reduce_shared_tile(const GemmArgs& g, const Seg& seg, int eidx, 
         const size_t unit_off = size_t(uu) * 1024 + size_t(e) * 4;
         int pc = owner;
         while (pc <= last) {
-            const float4* src[4];
-            int n = 0;
-            for (; pc <= last && n < 4; ++pc)
-                src[n++] = reinterpret_cast<const float4*>(g.ws_slots + size_t(pc) * WS_SLOT_FLOATS + unit_off);
-            float4 v[4];
+            const float* src = g.ws_slots + size_t(pc) * WS_SLOT_FLOATS + unit_off;
+            const int n = min(last + 1 - pc, 8);
+            float4 v[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (i < n) v[i] = __ldcg(src[i]);
+            for (int i = 0; i < 8; ++i)
+                if (i < n) v[i] = __ldcg(reinterpret_cast<const float4*>(src + i * WS_SLOT_FLOATS));
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 8; ++i)
                 if (i < n) { acc.x += v[i].x; acc.y += v[i].y; acc.z += v[i].z; acc.w += v[i].w; }
+            pc += n;
         }
         const int row = seg.a_row + q * 32 + (e & 31);
         const int col = (c < 4 ? seg.b_row0 + c * 32 : seg.b_row1 + (c - 4) * 32) + (e >> 5) * 4;
@@ -756,7 +806,7 @@ __device__ bool reduce_shared_tile(const GemmArgs& g, const Seg& seg, int eidx, 
 constexpr int GATHER_WARPS = 8, GATHER_GROUPS = 4;
 static_assert(GATHER_GROUPS == STAGES, "each gather group owns one ring slot");
 
-template <bool A_MN, bool B_MN, int GATHER = 0>
+template <bool A_MN, bool B_MN, int GATHER, bool SPLIT>
 __global__ void __launch_bounds__(GATHER ? GATHER_THREADS : GEMM_MAX_THREADS, 1)
 sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                        const __grid_constant__ CUtensorMap tmapC, const GemmArgs g) {
@@ -807,8 +857,11 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
     grid_dep_wait();
 
     const int n_ctas = gridDim.x, cta = blockIdx.x;
-    if (g.use_table) {
-        WorkIter it;
+    if (SPLIT) {
+        WorkIter<SPLIT> it;
+        it.split_prologue(g, cta, n_ctas, tab, threadIdx.x, blockDim.x);
+    } else if (g.use_table) {
+        WorkIter<SPLIT> it;
         it.init(g, cta, n_ctas, tab);
         if (it.tab) {                            // same decision in every thread and, below, in every role
             it.fill_table(g, tab, threadIdx.x, blockDim.x);
@@ -826,7 +879,7 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            WorkIter it;
+            WorkIter<SPLIT> it;
             it.init(g, cta, n_ctas, tab);
             Seg w;
             while (ok && it.next(g, w)) {
@@ -888,7 +941,7 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            WorkIter it;
+            WorkIter<SPLIT> it;
             it.init(g, cta, n_ctas, tab);
             Seg w;
             for (int seg = 0; ok && it.next(g, w); ++seg) {
@@ -955,7 +1008,7 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
             bool has_left, has_right;
         };
         // Walks the CTA's stages in the order every role sees them and stops at those of this group's slot.
-        WorkIter it;
+        WorkIter<SPLIT> it;
         it.init(g, cta, n_ctas, tab);
         Seg w;
         KIter kit;
@@ -1078,7 +1131,7 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
         const bool vec_ok = g.c_cs == 1 && (g.c_rs & 7) == 0 && aligned16;      // row-major result, 16-byte rows
         const bool vec_t_ok = g.c_rs == 1 && (g.c_cs & 7) == 0 && aligned16;    // column-major result
         zero_uncovered(g, vec_ok, vec_t_ok, etid, lane, epi_halves * cta + half, epi_halves * n_ctas);
-        WorkIter it;
+        WorkIter<SPLIT> it;
         it.init(g, cta, n_ctas, tab);
         int acc = 0;
         uint32_t acc_phase = 0;
@@ -1090,11 +1143,11 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
         int n_stores = 0;
         bool alive = true;
         while (alive && it.next(g, w)) {
-            const bool partial = w.parts > 1;
+            const bool partial = SPLIT && w.parts > 1;
             const bool ok = mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, g.status, ST_EPILOGUE);
             // Split launches synchronise all epilogue warps later (the shared tile), so they decide together whether
             // to go on; otherwise every warp decides for itself and no warp waits for the slowest one at every tile.
-            if (g.split ? !epilogue_all(ok, epi_threads) : !__all_sync(0xffffffffu, ok)) { alive = false; break; }
+            if (SPLIT ? !epilogue_all(ok, epi_threads) : !__all_sync(0xffffffffu, ok)) { alive = false; break; }
             tc_fence_after();
             const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quad * 32) << 16);
             const int row = w.a_row + etid;
@@ -1262,7 +1315,7 @@ sparsedrop_gemm_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_c
         }
         if (g.tma_store && lane == 0) bulk_wait_all();           // staged results are in global memory
         __syncwarp();
-        if (alive && has_shared) alive = reduce_shared_tile(g, shared, eidx, epi_threads, abort_flag);
+        if (SPLIT && alive && has_shared) alive = reduce_shared_tile(g, shared, eidx, epi_threads, abort_flag);
         __syncwarp();
     }
 
@@ -1425,8 +1478,8 @@ static int launch_pair(const CUtensorMap& tw, const CUtensorMap& ts, const CUten
     return SD_OK;
 }
 
-template <bool A_MN, bool B_MN, int GATHER = 0>
-static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmArgs& g, int grid,
+template <bool A_MN, bool B_MN, int GATHER, bool SPLIT>
+static int launch_schedule(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmArgs& g, int grid,
                           int epi_warps, cudaStream_t st) {
     // Called from the main thread and from autograd's worker threads at once: the per-device "already configured"
     // flags are atomics (setting the attribute twice is harmless, so relaxed ordering is enough).
@@ -1434,7 +1487,7 @@ static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CU
     int dev = 0;
     SD_CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev].load(std::memory_order_relaxed)) {
-        SD_CUDA_TRY(cudaFuncSetAttribute(sparsedrop_gemm_kernel<A_MN, B_MN, GATHER>,
+        SD_CUDA_TRY(cudaFuncSetAttribute(sparsedrop_gemm_kernel<A_MN, B_MN, GATHER, SPLIT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM));
         if (dev < 64) configured[dev].store(true, std::memory_order_relaxed);
     }
@@ -1448,8 +1501,14 @@ static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CU
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    SD_CUDA_TRY(cudaLaunchKernelEx(&cfg, sparsedrop_gemm_kernel<A_MN, B_MN, GATHER>, ta, tb, tc, g));
+    SD_CUDA_TRY(cudaLaunchKernelEx(&cfg, sparsedrop_gemm_kernel<A_MN, B_MN, GATHER, SPLIT>, ta, tb, tc, g));
     return SD_OK;
+}
+template <bool A_MN, bool B_MN, int GATHER = 0>
+static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmArgs& g, int grid, int epi_warps,
+                          cudaStream_t st) {
+    return g.split ? launch_schedule<A_MN, B_MN, GATHER, true>(ta, tb, tc, g, grid, epi_warps, st)
+                   : launch_schedule<A_MN, B_MN, GATHER, false>(ta, tb, tc, g, grid, epi_warps, st);
 }
 
 // SMs that the persistent grids of this library leave free (sd_set_sm_margin); SD_SM_MARGIN gives the initial value.
@@ -1611,6 +1670,7 @@ static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const v
     g.is_bf16 = dtype == SD_BF16;
     g.n_row_blocks = (M + 127) / 128;
     g.n_col_tiles = (N + BN - 1) / BN;
+    g.bn = BN;
     g.status = status;
     g.idesc256 = make_idesc(128, 256, g.is_bf16, a_mn, b_mn);
     g.idesc128 = make_idesc(128, 128, g.is_bf16, a_mn, b_mn);
@@ -1692,10 +1752,17 @@ static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const v
         const char* e = getenv("SD_SMALL_HALVES");         // tuning knob: 0 keeps whole 128x256 tiles on small launches
         return e ? atoi(e) : 1;
     }();
-    if (workspace && tiles_upper * 2 <= grid && k_tiles >= split_min_k_tiles && !c_panel_kg && !elementwise) {
+    if (workspace && tiles_upper * 2 <= grid && tiles_upper <= SPLIT_MAX_TILES && k_tiles >= split_min_k_tiles && !c_panel_kg && !elementwise) {
         if (reinterpret_cast<uintptr_t>(workspace) & 15) return fail(SD_ERR_LAYOUT, "workspace must be 16-byte aligned");
         if (grid > WS_MAX_CTAS) grid = WS_MAX_CTAS;
         g.split = 1;
+        // Tiles 128 wide where a tile's group would be large: every CTA parks and adds up half as many partial sums, and a
+        // stage of half the width costs two thirds of a full one, so the main loop loses little.  dW of (16384, 384, 384),
+        // 24 CTAs a tile: 18.4 -> 15.4 us; of (16384, 1536, 384), 8 CTAs a tile: 26.9 -> 31.
+        if (mode != MODE_SDD && !gather && N > 128 && tiles_upper * 16 <= grid) {
+            g.bn = 128;
+            g.n_col_tiles = (N + 127) / 128;
+        }
         g.ws_flags = static_cast<int*>(workspace);
         g.ws_slots = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + WS_FLAG_BYTES);
     } else if (small_halves && mode != MODE_SDD && !gather && N > 128 && tiles_upper * 2 <= grid) {
@@ -1707,17 +1774,12 @@ static int run_gemm(int mode, const void* A, int64_t a_rs, int64_t a_cs, const v
         grid = int(tiles_upper);
     }
     // Whole-tile launches describe their tiles once per CTA in shared memory when a tile's kept K tiles fit a 32-bit mask
-    // (and only when a CTA gets enough tiles for the table to pay: see TAB_MIN; the bound below counts every tile
-    // that may exist, the kernel checks the tiles that do)
-    // Short reductions (up to 16 K tiles) make a tile so short that resolving the next one between tiles shows: they get
-    // the table from five passes on ((16384, 1536, 384) forward: 25.3 -> 22.5 us); long ones only from TAB_MIN on, where
-    // the table's prologue would otherwise cost more than it saves (4096^3: +2.7 %).
-    static const int tab_min_short = [] {
-        const char* e = getenv("SD_TAB_MIN_SHORT");        // tuning knob: fewest passes that get the table, short reductions
-        return e ? atoi(e) : 5;
-    }();
-    g.tab_min = k_tiles <= 16 ? tab_min_short : TAB_MIN;
-    g.use_table = !g.split && (mode != MODE_DSD || k_tiles <= 32) && tiles_upper >= (long long)g.tab_min * grid / 2;
+    // and a CTA gets enough tiles for the table's barrier and its chain of index loads to pay: a DSD product from two passes on
+    // ((16384, 1536, 384) forward 21.3 -> 19.95 us against five), the others, whose tiles are found in two loads, from five
+    // (long reductions eight; with the table always, the dX of (512, 1024, 1024) took 9.85 us instead of 9.15).  The bound
+    // below counts every tile that may exist, the kernel checks the tiles that do.
+    g.tab_min = mode == MODE_DSD ? 2 : k_tiles <= 16 ? 5 : 8;
+    g.use_table = !g.split && (mode != MODE_DSD ? tiles_upper >= (long long)g.tab_min * grid / 2 : g.direct_mask != nullptr);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CUtensorMap tc = ta;
     if (c_panel_kg) {
