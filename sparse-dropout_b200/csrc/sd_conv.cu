@@ -145,7 +145,11 @@ __global__ void __launch_bounds__(kConvThreads) im2col_kept_s3_kernel(const unsi
 }
 
 // One CTA per kept block (grid-stride): 128 k-rows x 128 m-columns of colT.  Thread t owns the 8 consecutive m
-// starting at (t % 16) * 8 and visits k-rows (t / 16) + 16 * pass.
+// starting at (t % 16) * 8 and visits k-rows (t / 16) + 16 * pass.  Bound by instruction issue, so the pixels are decoded by one
+// division and counting on, and an element's address is the tap's pointer plus the pixel's offset (Off: 32 bits wherever
+// eight images fit them).  64 x 64 x 56 x 56, 3x3 stride 2, 40 MB written: 25.7 us, 33.6 with a division per pixel and a
+// 64-bit address per pixel and tap.
+template <class Off>
 __global__ void __launch_bounds__(kConvThreads) im2col_kept_kernel(const unsigned short* __restrict__ x,
                                                                    unsigned short* __restrict__ colT, ConvGeom g,
                                                                    const int* __restrict__ kept_pairs,
@@ -158,21 +162,22 @@ __global__ void __launch_bounds__(kConvThreads) im2col_kept_kernel(const unsigne
         const int kb = kept_pairs ? __ldg(kept_pairs + 2 * t + 1) : t - (t / g.Cb) * g.Cb;
         const int m0 = mb * 128 + mgrp * 8;
         if (m0 >= g.ldm) continue;
-        // decode the 8 output pixels once
-        long long base[8];
+        const int n0 = m0 / PQ, pq0 = m0 - n0 * PQ;
+        const unsigned short* image = x + (long long)n0 * g.C * HW;
+        Off off[8];                       // of the pixel's tap (0, 0) in channel 0, from the first pixel's image
         int hb[8], wb[8];
+        {
+            int p = pq0 / g.Q, q = pq0 - p * g.Q;
+            Off step = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int m = m0 + j;
-            if (m < g.M) {
-                const int n = m / PQ, pq = m - n * PQ, p = pq / g.Q, q = pq - p * g.Q;
-                base[j] = (long long)n * g.C * HW;
-                hb[j] = p * g.stride_h - g.pad_h;
+            for (int j = 0; j < 8; ++j) {
+                hb[j] = m0 + j < g.M ? p * g.stride_h - g.pad_h : -(1 << 28);   // never in range: padding columns are zero
                 wb[j] = q * g.stride_w - g.pad_w;
-            } else {
-                base[j] = 0;
-                hb[j] = -(1 << 28);   // never in range: the padding columns of colT are zero
-                wb[j] = 0;
+                off[j] = step + Off(p * g.stride_h - g.pad_h) * g.W + wb[j];
+                if (++q == g.Q) {
+                    q = 0;
+                    if (++p == g.P) { p = 0; step += Off(g.C) * HW; }
+                }
             }
         }
 #pragma unroll 2
@@ -181,13 +186,12 @@ __global__ void __launch_bounds__(kConvThreads) im2col_kept_kernel(const unsigne
             if (k >= g.K) break;
             const int c = k / RS, rs = k - c * RS, r = rs / g.S, s = rs - r * g.S;
             const int hoff = r * g.dil_h, woff = s * g.dil_w;
-            const unsigned short* xc = x + (long long)c * HW;
+            const unsigned short* tap = image + (long long)c * HW + (long long)hoff * g.W + woff;
             unsigned short v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const int h = hb[j] + hoff, w = wb[j] + woff;
-                const bool in = (unsigned)h < (unsigned)g.H && (unsigned)w < (unsigned)g.W;
-                v[j] = in ? __ldg(xc + base[j] + (long long)h * g.W + w) : (unsigned short)0;
+                const bool in = (unsigned)(hb[j] + hoff) < (unsigned)g.H && (unsigned)(wb[j] + woff) < (unsigned)g.W;
+                v[j] = in ? __ldg(tap + off[j]) : (unsigned short)0;
             }
             uint4 o;
             o.x = v[0] | (uint32_t(v[1]) << 16);
@@ -670,9 +674,13 @@ static int im2col_kept_impl(const void* x, int N, int C, int H, int W, int R, in
     else if (rows_path)
         sd::im2col_kept_rows_kernel<<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const unsigned short*>(x), static_cast<unsigned short*>(colT), g, pairs, n_kept);
-    else
-        sd::im2col_kept_kernel<<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    else {
+        // offsets span at most nine images and the padding around them
+        const bool small = (long long)C * H * W < (1ll << 27) && (long long)(pad_h + 1) * W < (1ll << 27) && pad_w < (1 << 27);
+        auto kernel = small ? &sd::im2col_kept_kernel<int> : &sd::im2col_kept_kernel<long long>;
+        kernel<<<grid, sd::kConvThreads, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const unsigned short*>(x), static_cast<unsigned short*>(colT), g, pairs, n_kept);
+    }
     SD_CUDA_TRY(cudaGetLastError());
     return SD_OK;
 }
