@@ -402,6 +402,10 @@ int sd_layernorm_bwd(const float* x, const void* dy, int dy_dtype, const float* 
 int sd_gelu_fwd(const void* x, void* y, int64_t n, int dtype, void* stream);
 int sd_gelu_bwd(const void* dy, const void* x, void* dx, int64_t n, int dtype, void* stream);
 
+/* y = x + r over n elements, x and y fp32, r of SD_F16 or SD_BF16 (the residual sums of the transformer consumers under autocast,
+ * eval/llm/model.py:80-83); all 16-byte aligned. */
+int sd_residual_add(const float* x, const void* r, float* y, int64_t n, int dtype, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * AdamW over all parameters of a model in one launch (the reference trains with torch.optim.AdamW(fused=True),
  * eval/llm/model.py:157-173).  Every tensor is contiguous fp32 in device memory, 16-byte aligned; `step` is its step counter

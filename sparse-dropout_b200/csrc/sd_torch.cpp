@@ -853,6 +853,39 @@ std::optional<Tensor> gelu(const Tensor& x) {
     return y;
 }
 
+// ---------------------------------------------------------------- residual sum
+struct SparseDropResidualBackward : public Node {
+    at::ScalarType r_type = at::kHalf;
+
+    std::string name() const override { return "SparseDropResidualBackward"; }
+    variable_list apply(variable_list&& grads) override {
+        const Tensor& dy = grads[0];
+        if (!dy.defined()) return {Tensor(), Tensor()};
+        return {dy, task_should_compute_output(1) ? dy.to(r_type) : Tensor()};
+    }
+};
+
+// x + r, or nothing if the kernel does not serve these tensors: plain contiguous ones of one shape, x in fp32, r in 16 bits.
+std::optional<Tensor> residual_add(const Tensor& x, const Tensor& r) {
+    py::gil_scoped_release no_gil;
+    const at::ScalarType t = r.scalar_type();
+    if (!x.is_cuda() || x.scalar_type() != at::kFloat || (t != at::kHalf && t != at::kBFloat16) || r.device() != x.device() ||
+        at::isTensorSubclassLike(x) || at::isTensorSubclassLike(r) || x.sizes() != r.sizes() || !x.numel() || !x.is_contiguous() ||
+        !r.is_contiguous() || !aligned16(x) || !aligned16(r) || torch::autograd::isFwGradDefined(x) || torch::autograd::isFwGradDefined(r))
+        return std::nullopt;
+    const at::Device dev = x.device();
+    c10::cuda::OptionalCUDAGuard guard(dev);
+    Tensor y = at::detail::empty_cuda(x.sizes(), at::kFloat, dev, std::nullopt);
+    check_rc(sd_residual_add(x.data_ptr<float>(), r.data_ptr(), y.data_ptr<float>(), x.numel(), dtype_code(t),
+                             c10::cuda::getCurrentCUDAStream(dev.index()).stream()));
+    if (!torch::autograd::compute_requires_grad(x, r)) return y;
+    std::shared_ptr<SparseDropResidualBackward> node(new SparseDropResidualBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, r));
+    node->r_type = t;
+    torch::autograd::set_history(y, node);
+    return y;
+}
+
 // ---------------------------------------------------------------- AdamW
 // The tensors of one optimizer, described to the kernel once; a step checks that none of them has moved since.  Only weak
 // references are held: parameters lead back to whoever holds this object (their gradient hooks), and Python's collector
@@ -928,6 +961,7 @@ PYBIND11_MODULE(sd_torch, m) {
     m.def("gemm_sdd", &gemm_sdd);
     m.def("layer_norm", &layer_norm);
     m.def("gelu", &gelu);
+    m.def("residual_add", &residual_add);
     py::class_<AdamW>(m, "AdamW")
         .def(py::init<const std::vector<std::array<Tensor, 5>>&, const std::vector<int64_t>&>())
         .def("step", &AdamW::step);

@@ -31,7 +31,7 @@ EXPORTS = (
     "sd_gemm_dsd_relu", "sd_gemm_dsd_f32", "sd_gemm_sdd_relu_mask", "sd_gemm_sdd_f32", "sd_cast16",
     "sd_plan_batch_desc_bytes", "sd_plan_batch_describe", "sd_plan_batch_launch", "sd_set_sm_margin",
     "sd_layernorm_fwd", "sd_layernorm_bwd_workspace_bytes", "sd_layernorm_bwd",
-    "sd_gelu_fwd", "sd_gelu_bwd",
+    "sd_gelu_fwd", "sd_gelu_bwd", "sd_residual_add",
     "sd_adamw_table_bytes", "sd_adamw_table_fill", "sd_adamw_step",
 )
 
@@ -107,6 +107,8 @@ def lib() -> C.CDLL:
     L.sd_gemm_sdd_relu_mask.argtypes = mat * 3 + [i32, i32, i32, vp, vp, i64, f32, i32, vp, vp, vp]
     L.sd_gemm_sdd_f32.restype = i32
     L.sd_gemm_sdd_f32.argtypes = L.sd_gemm_sdd_relu_mask.argtypes
+    L.sd_residual_add.restype = i32
+    L.sd_residual_add.argtypes = [vp, vp, vp, i64, i32, vp]
     L.sd_gelu_fwd.restype = i32
     L.sd_gelu_fwd.argtypes = [vp, vp, i64, i32, vp]
     L.sd_gelu_bwd.restype = i32

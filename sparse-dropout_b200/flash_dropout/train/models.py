@@ -17,6 +17,7 @@ from torch import nn
 from flash_dropout.layers import DropoutMM
 from flash_dropout.layers.gelu import GELU
 from flash_dropout.layers.norm import LayerNorm
+from flash_dropout.layers.residual import residual_add
 
 
 def next_multiple(x: int, base: int) -> int:
@@ -85,8 +86,8 @@ class Block(nn.Module):
         self.mlp = MLP(n_embed, dropout)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        x = x + self.attn(self.ln_1(x))
-        return x + self.mlp(self.ln_2(x))
+        x = residual_add(x, self.attn(self.ln_1(x)))
+        return residual_add(x, self.mlp(self.ln_2(x)))
 
 
 class GPT(nn.Module):
@@ -172,8 +173,8 @@ class ViTTransformer(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         for attn, ff in self.layers:
-            x = attn(x) + x
-            x = ff(x) + x
+            x = residual_add(x, attn(x))
+            x = residual_add(x, ff(x))
         return self.norm(x)
 
 
