@@ -193,3 +193,14 @@ def test_functional_mask_is_fresh_on_graph_replay(built_lib):
     finally:
         sd_random.disable_device_counter()
         sd_random.follow_torch_seed()
+
+
+@pytest.mark.parametrize("R,C", [(32, 32), (32, 1), (1, 32), (31, 17), (33, 32), (32, 33)])
+@pytest.mark.parametrize("p", [0.0, 0.5, 1.0])
+def test_plan_of_one_warp_per_row(built_lib, R, C, p):
+    """Up to 32 x 32 tiles a warp draws a row and writes a column: the largest such grid, its neighbours, nothing and
+    everything dropped."""
+    from flash_dropout.cuda.binding_gemm import BlockPlan
+    mask = torch.rand(R, C, generator=torch.Generator().manual_seed(R * 37 + C)) < p
+    plan = BlockPlan.from_mask(mask.to("cuda:0"), R * 128, C * 128, 128)
+    _check_plan(plan, mask.numpy(), R * 128, C * 128, 128)
