@@ -523,7 +523,7 @@ def run_ours(args) -> None:
                                   if world > 1 else "")},
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak, "traffic": NCU_TRAFFIC_BYTES_PER_LAUNCH,
-                         "kernel": "sparsedrop_gemm_kernel (3 launches per step: DSD fwd, SDD dX, DSD dW)",
+                         "kernel": "sparsedrop_pair_kernel (3 launches per step: DSD fwd, SDD dX, DSD dW)",
                          "peak_source": peak_src, "frac_of_nominal_2250": achieved / 2250.0,
                          "avg_launch_ms": {"dsd_fwd": per_kernel_ms[0], "sdd_dx": per_kernel_ms[1], "dsd_dw": per_kernel_ms[2]},
                          "flops_per_launch": useful_flops(kept) / 3 / steps},
