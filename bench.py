@@ -46,9 +46,9 @@ METRIC = "DSD/SDD useful TFLOP/s (DSD fwd + SDD dX + DSD dW on kept 128x128 bloc
 WORKLOAD = ("SparseDrop linear fwd+bwd, M=N=K=4096, fp16 in / fp32 acc, 128x128 blocks, "
             "p=0.5, x,W,dy~N(0,K^-1/2), per-step Philox mask (seed 0, offset=step)")
 # DRAM bytes (read + written) per GEMM launch of this workload as an ncu capture counts them: the mean of the
-# step's three launches, 60.3 / 92.2 / 63.1 MB.  A profiler figure cannot be taken inside a timed run, so it is
+# step's three launches, 59.8 / 93.1 / 56.0 MB.  A profiler figure cannot be taken inside a timed run, so it is
 # carried here as a constant and reported as `roofline.traffic`.
-NCU_TRAFFIC_BYTES_PER_LAUNCH = 71.9e6
+NCU_TRAFFIC_BYTES_PER_LAUNCH = 69.6e6
 
 
 def measured_peaks() -> tuple[float, str]:
