@@ -195,37 +195,6 @@ void cast_pair(const Tensor& a, Tensor& a16, const Tensor& b, Tensor& b16, at::S
                            dtype_code(dt), stream));
 }
 
-// The copy of the last activation this thread cast, for consecutive layers that are fed the very same tensor (the q / k / v
-// projections of an attention block).  A layer sees a fresh 2-D view on every call, so the tensor is identified by the one
-// that owns its memory plus the view's geometry and version; only weak references are held, so an entry dies with its
-// tensor and keeps no memory alive.
-struct CastEntry {
-    c10::weak_intrusive_ptr<c10::TensorImpl> owner, copy;
-    uint32_t version;
-    at::ScalarType dt;
-    int64_t offset;
-    std::vector<int64_t> size, stride;
-    cudaStream_t stream;
-};
-struct CastCache {
-    std::optional<CastEntry> e;
-    static Tensor owner_of(const Tensor& x) { return x.is_view() ? Tensor(x._base()) : x; }
-    Tensor find(const Tensor& x, at::ScalarType dt, cudaStream_t stream) {
-        if (!e || x.is_inference() || e->dt != dt || e->stream != stream || e->version != x._version() || e->offset != x.storage_offset()) return {};
-        if (x.sizes() != at::IntArrayRef(e->size) || x.strides() != at::IntArrayRef(e->stride)) return {};
-        auto own = e->owner.lock();
-        if (!own || own.get() != owner_of(x).unsafeGetTensorImpl()) return {};
-        auto copy = e->copy.lock();
-        return copy ? Tensor(std::move(copy)) : Tensor();
-    }
-    void put(const Tensor& x, const Tensor& x16, cudaStream_t stream) {
-        if (x.is_inference()) return;
-        e.emplace(CastEntry{c10::weak_intrusive_ptr<c10::TensorImpl>(owner_of(x).getIntrusivePtr()),
-                            c10::weak_intrusive_ptr<c10::TensorImpl>(x16.getIntrusivePtr()), uint32_t(x._version()), x16.scalar_type(),
-                            x.storage_offset(), x.sizes().vec(), x.strides().vec(), stream});
-    }
-};
-
 // ---------------------------------------------------------------- a SparseDrop linear
 struct PyCallback {
     PyObject* f;
@@ -359,14 +328,12 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
         if (input.scalar_type() != dt && input.scalar_type() != at::kFloat) input = input.to(dt);
         if (!lowp && weight.scalar_type() != dt && weight.scalar_type() != at::kFloat) weight = weight.to(dt);
         at::NoGradGuard no_grad;
-        static thread_local CastCache cache;
         const bool cast_x = input.scalar_type() != dt, cast_w = !lowp && weight.scalar_type() != dt;
         x16 = input;
         w16 = lowp ? *weight_lowp : weight;
-        if (cast_x) x16 = cache.find(input, dt, L.stream);
-        const bool hit = x16.defined();
-        if (!hit || cast_w) cast_pair(hit ? Tensor() : input, x16, cast_w ? weight : Tensor(), w16, dt, L.stream);
-        if (!hit) cache.put(input, x16, L.stream);
+        // Every call casts for itself: a copy kept from an earlier call could not be known to be current, as a CUDA graph's
+        // replay rewrites tensors without a sign that the host could see, and a copy made during a capture holds nothing yet.
+        if (cast_x || cast_w) cast_pair(cast_x ? input : Tensor(), x16, cast_w ? weight : Tensor(), w16, dt, L.stream);
     } else {
         x16 = input;
         w16 = weight;

@@ -28,7 +28,6 @@ from flash_dropout import _lib
 from flash_dropout import random as sd_random
 from flash_dropout.cuda.binding_gemm import BlockPlan, PlanBatch, _on_device, _rep
 
-from .blockwise_dropout_matmul_cuda import _autocast_input
 from .im2col_conv2d import conv_output_size
 
 
@@ -110,7 +109,7 @@ def blockwise_dropout_conv2d(input: torch.Tensor, kernel: torch.Tensor, block_si
         # fp32 tensors are cast inside the operator and get their gradients in fp32; others by autograd
         dt = torch.get_autocast_dtype("cuda")
         if input.dtype not in (dt, torch.float32):
-            input = _autocast_input(input, dt)
+            input = input.to(dt)
         if kernel.dtype not in (dt, torch.float32):
             kernel = kernel.to(dt)
     padding, stride, dilation = tuple(padding), tuple(stride), tuple(dilation)

@@ -25,13 +25,17 @@ _last_cast = {"key": None, "src": None, "ref": None}
 
 
 def _autocast_input(input: torch.Tensor, dt: torch.dtype) -> torch.Tensor:
-    """``input.to(dt)``, shared between consecutive layers that are fed the very same tensor (the q / k / v
-    projections of an attention block): one cast forward, and one cast of the summed gradient backward.
+    """``input.to(dt)``, shared between consecutive calls with the very same tensor: one cast for the q / k / v projections
+    of an attention block, and one cast of the summed gradient backward.
 
-    The entry is valid only for the very tensor it was made from, unmodified since.  A layer sees a fresh 2-D
-    view object on every call, so the tensor is identified by the object that owns its memory (the view's base)
-    plus the view's geometry; the entry holds only a weak reference to that owner, so once it is freed the entry
-    is dead and a new tensor that the allocator places at the same address can never be taken for it."""
+    For callers that know that nothing but torch operators writes ``input``.  The operators cast for themselves instead: a
+    CUDA graph's replay rewrites tensors without advancing their version, and a copy made during a capture holds nothing
+    before the first replay.
+
+    The entry is valid only for the very tensor it was made from, unmodified since.  The tensor is identified by the object
+    that owns its memory (a view's base) plus the view's geometry; the entry holds only a weak reference to that owner, so
+    once it is freed the entry is dead and a new tensor that the allocator places at the same address can never be taken
+    for it."""
     if input.dtype == dt:
         return input
     owner = input._base if input._base is not None else input
@@ -101,7 +105,7 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
         # fp32 operands are cast inside the operator; others by autograd
         dt = torch.get_autocast_dtype("cuda")
         if input.dtype not in (dt, torch.float32):
-            input = _autocast_input(input, dt)
+            input = input.to(dt)
     target, accumulate, notify = wgrad if wgrad is not None else (None, False, None)
     try:
         return _lib.ext().linear(input, weight, buf, R, C, rep_r, rep_c, not isinstance(block_size, int), p, seed, offset,
