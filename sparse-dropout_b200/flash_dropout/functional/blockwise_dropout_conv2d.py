@@ -29,6 +29,7 @@ from flash_dropout import random as sd_random
 from flash_dropout.cuda.binding_gemm import BlockPlan, PlanBatch, _on_device, _rep
 
 from .im2col_conv2d import conv_output_size
+from .recorded import recorded
 
 
 def _round8(v: int) -> int:
@@ -105,6 +106,13 @@ def blockwise_dropout_conv2d(input: torch.Tensor, kernel: torch.Tensor, block_si
     column of padding, rows of 8..64 pixels) never materialise the im2col matrix; others, and ``fused=False``, go
     through the kept-block im2col stage."""
     assert 0 <= p < 1, "Dropout probability must be in [0, 1)"
+    if torch.jit.is_tracing():
+        return recorded(lambda x, k: _conv2d(x, k, block_size, p, padding, stride, dilation, plan, recompute_cols, fused), input,
+                        kernel)
+    return _conv2d(input, kernel, block_size, p, padding, stride, dilation, plan, recompute_cols, fused)
+
+
+def _conv2d(input, kernel, block_size, p, padding, stride, dilation, plan, recompute_cols, fused) -> torch.Tensor:
     if torch.is_autocast_enabled("cuda"):
         # fp32 tensors are cast inside the operator and get their gradients in fp32; others by autograd
         dt = torch.get_autocast_dtype("cuda")

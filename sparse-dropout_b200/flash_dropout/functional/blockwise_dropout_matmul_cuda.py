@@ -20,6 +20,7 @@ from flash_dropout import _lib
 from flash_dropout import random as sd_random
 from flash_dropout.cuda.binding_gemm import BlockPlan, PlanBatch, _rep
 
+from .recorded import recorded
 
 _last_cast = {"key": None, "src": None, "ref": None}
 
@@ -80,6 +81,15 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
       any_rank        ``input`` may have any number of leading dimensions, all of them rows.
     """
     assert 0 <= p < 1, "Dropout probability must be in [0, 1)"
+    if torch.jit.is_tracing():
+        return recorded(lambda x, w: _matmul(x, w, block_size, p, plan, relu, input_relu, grad_premasked, wgrad,
+                                             recompute_plan, None, any_rank), input, weight)
+    return _matmul(input, weight, block_size, p, plan, relu, input_relu, grad_premasked, wgrad, recompute_plan, weight_lowp,
+                   any_rank)
+
+
+def _matmul(input, weight, block_size, p, plan, relu, input_relu, grad_premasked, wgrad, recompute_plan, weight_lowp,
+            any_rank) -> torch.Tensor:
     rep_r, rep_c = _rep(block_size)
     seed = offset = 0
     counter = None

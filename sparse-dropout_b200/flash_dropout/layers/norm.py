@@ -5,7 +5,7 @@ Same module as ``torch.nn.LayerNorm`` (same parameters and ``state_dict`` keys; 
 On a CUDA fp32 input whose normalised width is a multiple of 4 up to 1024 the forward is one pass that writes its
 result in the dtype the consumer reads (the autocast dtype when autocast is on, so the separate cast disappears) and
 the backward one pass for dx plus a small reduction for the parameter gradients; everything else (CPU tensors, other
-dtypes, wider rows, several normalised dimensions) goes to ``F.layer_norm`` unchanged.
+dtypes, wider rows, several normalised dimensions, a trace being recorded) goes to ``F.layer_norm`` unchanged.
 """
 from __future__ import annotations
 
@@ -14,9 +14,10 @@ import torch.nn.functional as F
 
 from flash_dropout import _lib
 
+
 def layer_norm(x: torch.Tensor, normalized_shape, weight, bias, eps: float) -> torch.Tensor:
     """``F.layer_norm`` with the fused path where it applies (see the module docstring)."""
-    if len(normalized_shape) == 1 and weight is not None and x.is_cuda:
+    if len(normalized_shape) == 1 and weight is not None and x.is_cuda and not torch.jit.is_tracing():
         y = _lib.ext().layer_norm(x, weight, bias, eps)       # csrc/sd_torch.cpp: forward launch and autograd node
         if y is not None:
             return y
