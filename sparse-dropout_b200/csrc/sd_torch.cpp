@@ -229,7 +229,7 @@ struct SparseDropLinearBackward : public Node {
     bool pair_block = false;
     int64_t M = 0, K = 0, N = 0;
     std::vector<int64_t> lead;                     // shape of an input that is not 2-D
-    double p = 0;
+    double p = 0, draw_p = 0;                      // of the scale, and of the draw
     bool x_f32 = false, w_f32 = false;             // the layer's own tensors are fp32: their gradients leave in fp32
     Options opt;
 
@@ -296,12 +296,13 @@ variable_list SparseDropLinearBackward::gradients(variable_list&& grads) {
 
 // y = (keep o input) . weight^T / (1 - p) of 2-D CUDA tensors, see blockwise_dropout_matmul in
 // functional/blockwise_dropout_matmul_cuda.py for the meaning of the arguments.  `plan` with its grid, or none: drawn from
-// (seed, offset) and the optional device counter.  `recompute`: (seed, offset) are all that is kept for backward.
+// (seed, offset) and the optional device counter with blocks of rep_r x rep_c tiles at draw_p.  `recompute`: what it is drawn
+// from is all that is kept for backward.  `p` is the scale's.
 Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<Tensor>& plan_, int64_t plan_R, int64_t plan_C,
               int64_t rep_r, int64_t rep_c, bool pair_block, double p, uint64_t seed, uint64_t offset,
               const std::optional<Tensor>& counter, bool relu, bool input_relu, bool premasked,
               const std::optional<Tensor>& wgrad, bool wgrad_acc, py::handle notify, bool recompute,
-              const std::optional<Tensor>& weight_lowp, bool any_rank) {
+              const std::optional<Tensor>& weight_lowp, bool any_rank, double draw_p) {
     Options opt;
     opt.relu = relu;
     opt.input_relu = input_relu;
@@ -373,7 +374,7 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
         d.counter = counter && counter->defined() ? static_cast<uint64_t*>(counter->data_ptr()) : nullptr;
         d.rep_r = int(rep_r);
         d.rep_c = int(rep_c);
-        d.p = float(p);
+        d.p = float(draw_p);
         if (!plan.defined()) plan = draw_plan(d, M, K, dev, L.stream);
         if (input.dim() == 2)
             out = empty2(M, N, xs.scalar_type(), dev);
@@ -398,6 +399,7 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     node->block_m = rep_r * TILE;
     node->block_k = rep_c * TILE;
     node->pair_block = pair_block;
+    node->draw_p = draw_p;
     if (!recompute || d.counter) node->plan = plan;
     node->M = M;
     node->K = K;
@@ -426,7 +428,7 @@ PyObject* get_origin(PyObject* self, void*) {
     const auto* n = node_of(self);
     if (n->plan.defined()) Py_RETURN_NONE;
     py::object block = n->pair_block ? py::object(py::make_tuple(n->block_m, n->block_k)) : py::object(py::int_(n->block_m));
-    return py::make_tuple(n->M, n->K, block, n->p, n->draw.seed, n->draw.offset).release().ptr();
+    return py::make_tuple(n->M, n->K, block, n->draw_p, n->draw.seed, n->draw.offset).release().ptr();
 }
 void register_node() {
     using namespace torch::autograd;

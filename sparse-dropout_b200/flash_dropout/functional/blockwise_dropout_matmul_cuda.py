@@ -73,8 +73,9 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
                       is called afterwards;
       recompute_plan  keep only (seed, offset) of the mask between forward and backward and draw the plan again there
                       (one more plan launch per layer in backward; the plan buffer, 4 bytes per tile and list entry, is
-                      not kept alive).  Applies to plans drawn from a host-side offset; a plan whose offset was read
-                      from the device-side counter (CUDA-graph mode, where plan buffers are static anyway) is kept;
+                      not kept alive).  Applies to plans drawn from a host-side offset, a given one with the block size
+                      and p it was drawn with; a plan whose offset was read from the device-side counter (CUDA-graph
+                      mode, where plan buffers are static anyway) is kept;
       weight_lowp     an up-to-date copy of ``weight`` in the autocast dtype that the caller keeps (a training step that
                       casts all weights with one launch): used instead of casting again, which needs ``wgrad`` (the copy
                       is outside autograd, so the weight gradient has to leave through the fused store);
@@ -91,6 +92,7 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
 def _matmul(input, weight, block_size, p, plan, relu, input_relu, grad_premasked, wgrad, recompute_plan, weight_lowp,
             any_rank) -> torch.Tensor:
     rep_r, rep_c = _rep(block_size)
+    draw_p = p
     seed = offset = 0
     counter = None
     fresh = False
@@ -108,7 +110,10 @@ def _matmul(input, weight, block_size, p, plan, relu, input_relu, grad_premasked
     else:
         buf, R, C = plan.buf, plan.R, plan.C
         if recompute_plan and plan.origin is not None:
-            seed, offset = plan.origin[4:]
+            # backward draws this very plan again, whatever block size and p the call names
+            _, _, block_size, draw_p, seed, offset = plan.origin
+            rep_r, rep_c = _rep(block_size)
+            seed, offset = seed & (2**64 - 1), offset & (2**64 - 1)
         else:
             recompute_plan = False
     if torch.is_autocast_enabled("cuda"):
@@ -120,7 +125,7 @@ def _matmul(input, weight, block_size, p, plan, relu, input_relu, grad_premasked
     try:
         return _lib.ext().linear(input, weight, buf, R, C, rep_r, rep_c, not isinstance(block_size, int), p, seed, offset,
                                 counter, relu, input_relu, grad_premasked, target, accumulate, notify, recompute_plan,
-                                weight_lowp, any_rank)
+                                weight_lowp, any_rank, draw_p)
     except Exception:
         if fresh:
             sd_random.give_back(offset)        # a call that was refused has used no mask

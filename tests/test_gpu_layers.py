@@ -328,3 +328,24 @@ def test_weight_shadows_equal_per_layer_casts_and_are_ignored_when_stale(built_l
             outs.append(model(x))
     assert torch.equal(outs[0], outs[1])
     sd_random.follow_torch_seed()
+
+
+@pytest.mark.parametrize("drawn,called", [((256, 0.5), (128, 0.5)), ((128, 0.25), (128, 0.5)), (((128, 256), 0.5), (256, 0.5))])
+def test_recompute_plan_redraws_the_plan_it_was_given(built_lib, drawn, called):
+    """A drawn plan handed to a call that names another block size or p: the mask is the plan's, forward and backward,
+    whether it is kept or drawn again; the call's p is the scale."""
+    import flash_dropout.functional as F
+    from flash_dropout.cuda.binding_gemm import BlockPlan
+    g = torch.Generator(device=DEV).manual_seed(8)
+    x, w, dy = (torch.randn(*s, generator=g, device=DEV).half() for s in ((640, 1024), (256, 1024), (640, 256)))
+    outs = []
+    for recompute in (False, True):
+        plan = BlockPlan.from_seed(640, 1024, drawn[0], drawn[1], -5, 2, DEV)
+        xa, wa = x.clone().requires_grad_(), w.clone().requires_grad_()
+        y = F.cuda_blockwise_dropout_matmul(xa, wa, called[0], called[1], plan=plan, recompute_plan=recompute)
+        if recompute:
+            assert y.grad_fn.plan is None and y.grad_fn.origin == (*plan.origin[:4], 2**64 - 5, 2)
+        y.backward(dy)
+        outs.append((y.detach(), xa.grad, wa.grad))
+    for a, b, name in zip(outs[0], outs[1], ("y", "dx", "dw")):
+        assert torch.equal(a, b), name
