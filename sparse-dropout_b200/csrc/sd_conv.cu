@@ -600,15 +600,15 @@ static int make_geom(ConvGeom* g, int N, int C, int H, int W, int R, int S, int 
         return fail(SD_ERR_INVALID_ARG, "conv sizes must be positive");
     if (stride_h <= 0 || stride_w <= 0 || dil_h <= 0 || dil_w <= 0 || pad_h < 0 || pad_w < 0)
         return fail(SD_ERR_INVALID_ARG, "stride and dilation must be positive, padding non-negative");
-    const int P = (H + 2 * pad_h - dil_h * (R - 1) - 1) / stride_h + 1;
-    const int Q = (W + 2 * pad_w - dil_w * (S - 1) - 1) / stride_w + 1;
-    if (P <= 0 || Q <= 0) return fail(SD_ERR_INVALID_ARG, "the filter does not fit the padded input");
-    const long long M = (long long)N * P * Q, K = (long long)C * R * S;
+    const long long over_h = H + 2ll * pad_h - (long long)dil_h * (R - 1) - 1, over_w = W + 2ll * pad_w - (long long)dil_w * (S - 1) - 1;
+    if (over_h < 0 || over_w < 0) return fail(SD_ERR_INVALID_ARG, "the filter does not fit the padded input");
+    const long long P = over_h / stride_h + 1, Q = over_w / stride_w + 1;
+    const long long M = N * P * Q, K = (long long)C * R * S;
     if (M > (1ll << 30) || K > (1ll << 30)) return fail(SD_ERR_TOO_LARGE, "im2col matrix too large (M=%lld, K=%lld)", M, K);
     if (panels) ldm = ((M + 127) / 128) * 128;      // whole panels exist
     if (ldm < M || (ldm & 7)) return fail(SD_ERR_LAYOUT, "ldm (%lld) must be >= N*P*Q (%lld) and a multiple of 8", (long long)ldm, M);
     if (k_gemm < K) return fail(SD_ERR_INVALID_ARG, "k_gemm (%d) must be >= C*R*S (%lld)", k_gemm, K);
-    *g = ConvGeom{N, C, H, W, R, S, P, Q, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, int(M), int(K), ldm,
+    *g = ConvGeom{N, C, H, W, R, S, int(P), int(Q), pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, int(M), int(K), ldm,
                   int((M + 127) / 128), (k_gemm + 127) / 128, panels ? 128 : ldm, panels ? (long long)k_gemm * 128 : 0};
     return SD_OK;
 }

@@ -1924,8 +1924,9 @@ int sd_conv_fused_supported(int N, int C, int H, int W, int R, int S, int pad_h,
     if (N <= 0 || C <= 0 || H <= 0 || W <= 0 || R <= 0 || S != 3) return 0;
     if (stride_w != 1 || dil_w != 1 || pad_w != 1 || stride_h <= 0 || dil_h <= 0 || pad_h < 0) return 0;
     if (W != 8 && W != 16 && W != 32 && W != 64) return 0;
-    const long long P = ((long long)H + 2 * pad_h - (long long)dil_h * (R - 1) - 1) / stride_h + 1;
-    if (P <= 0) return 0;
+    const long long over = H + 2ll * pad_h - (long long)dil_h * (R - 1) - 1;
+    if (over < 0) return 0;                                   // the filter is higher than the padded input
+    const long long P = over / stride_h + 1;
     if ((long long)N * P * W > (1ll << 30) || (long long)C * R * 3 > (1ll << 30)) return 0;
     if ((long long)N * C * H * W > (1ll << 31) - 1) return 0;
     return 1;

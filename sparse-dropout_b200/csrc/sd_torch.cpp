@@ -610,11 +610,15 @@ Tensor conv2d(const Tensor& input_, const Tensor& kernel_, const std::optional<T
     g.Ko = int(kernel.size(0)); g.R = int(kernel.size(2)); g.S = int(kernel.size(3));
     if (kernel.size(1) != g.C) bad("kernel expects " + std::to_string(kernel.size(1)) + " input channels, input has " + std::to_string(g.C));
     g.ph = int(padding[0]); g.pw = int(padding[1]); g.sh = int(stride[0]); g.sw = int(stride[1]); g.dh = int(dilation[0]); g.dw = int(dilation[1]);
-    if (g.sh <= 0 || g.sw <= 0) bad("stride must be positive");
-    g.P = (g.H + 2 * g.ph - g.dh * (g.R - 1) - 1) / g.sh + 1;
-    g.Q = (g.W + 2 * g.pw - g.dw * (g.S - 1) - 1) / g.sw + 1;
+    if (g.sh <= 0 || g.sw <= 0 || g.dh <= 0 || g.dw <= 0) bad("stride and dilation must be positive");
+    // rows and columns that the filter can move over; negative: it is larger than the padded input
+    const int64_t over_h = int64_t(g.H) + 2 * int64_t(g.ph) - int64_t(g.dh) * (g.R - 1) - 1;
+    const int64_t over_w = int64_t(g.W) + 2 * int64_t(g.pw) - int64_t(g.dw) * (g.S - 1) - 1;
+    if (over_h < 0 || over_w < 0) bad("the filter does not fit the padded input");
+    g.P = int(over_h / g.sh + 1);
+    g.Q = int(over_w / g.sw + 1);
     const int64_t M = int64_t(g.N) * g.P * g.Q, K = int64_t(g.C) * g.R * g.S;
-    if (g.P <= 0 || g.Q <= 0 || M > (1ll << 30) || K > (1ll << 30)) bad("the filter does not fit the padded input, or the im2col matrix is too large");
+    if (M > (1ll << 30) || K > (1ll << 30)) bad("the im2col matrix is too large");
     g.M = int(M);
     g.K = int(K);
     g.Kg = (g.K + 63) & ~63;                        // the im2col matrix is kept in panels: k extent a multiple of 64
