@@ -596,6 +596,7 @@ Tensor conv2d(const Tensor& input_, const Tensor& kernel_, const std::optional<T
               bool want_fused) {
     py::gil_scoped_release no_gil;
     if (!input_.is_cuda() || !kernel_.is_cuda()) bad("input and kernel must be CUDA");
+    if (input_.device() != kernel_.device()) bad("input and kernel must be on the same device");
     no_forward_ad("SparseDropConv2d", {input_, kernel_});
     const Tensor &input = input_, &kernel = kernel_;
     const bool amp = at::autocast::is_autocast_enabled(at::kCUDA);
