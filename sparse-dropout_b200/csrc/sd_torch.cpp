@@ -179,6 +179,10 @@ Tensor draw_plan(const Draw& d, int64_t M, int64_t K, const at::Device& dev, cud
     return buf;
 }
 
+void check_plan_device(const std::optional<Tensor>& plan, const at::Device& dev) {
+    if (plan && plan->defined() && plan->device() != dev) bad("the plan must be on the device of the operands");
+}
+
 // ---------------------------------------------------------------- casts under autocast
 inline bool flat_f32(const Tensor& t) {
     return t.scalar_type() == at::kFloat && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
@@ -318,14 +322,18 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     if (input_.device() != weight_.device()) bad("A and B must be on the same device");
     no_forward_ad("SparseDropLinear", {input_, weight_});
     const at::Device dev = input_.device();
+    const bool amp = at::autocast::is_autocast_enabled(at::kCUDA);
+    const at::ScalarType amp_t = amp ? at::autocast::get_autocast_dtype(at::kCUDA) : at::kFloat;
+    const bool lowp = amp && weight_lowp && opt.wgrad.defined() && weight_lowp->scalar_type() == amp_t && weight_lowp->sizes() == weight_.sizes();
+    if (lowp && weight_lowp->device() != dev) bad("A and B must be on the same device");
+    check_plan_device(plan_, dev);
     c10::cuda::OptionalCUDAGuard guard(dev);
     const Launch L(dev);
 
     // operands in 16 bits; fp32 ones are cast here, outside autograd, and their gradients leave in fp32
     Tensor input = input_, weight = weight_, x16, w16;
-    if (at::autocast::is_autocast_enabled(at::kCUDA)) {
-        const at::ScalarType dt = at::autocast::get_autocast_dtype(at::kCUDA);
-        const bool lowp = weight_lowp && opt.wgrad.defined() && weight_lowp->scalar_type() == dt && weight_lowp->sizes() == weight.sizes();
+    if (amp) {
+        const at::ScalarType dt = amp_t;
         if (input.scalar_type() != dt && input.scalar_type() != at::kFloat) input = input.to(dt);
         if (!lowp && weight.scalar_type() != dt && weight.scalar_type() != at::kFloat) weight = weight.to(dt);
         at::NoGradGuard no_grad;
@@ -458,6 +466,9 @@ int check_pair(const Tensor& A, const Tensor& B) {
     if (A.device() != B.device()) bad("A and B must be on the same device");
     return dtype_code(A.scalar_type());
 }
+void check_mask_device(const Tensor& mask, const Tensor& A) {
+    if (mask.is_cuda() && mask.device() != A.device()) bad("Mask must be on the operands' device");
+}
 Tensor plan_from_mask(const Tensor& mask, int64_t rows, int64_t cols, int64_t rep_r, int64_t rep_c, cudaStream_t stream) {
     if (mask.scalar_type() != at::kBool) bad("Mask must be bool");
     if (!mask.is_cuda() || mask.dim() != 2) bad("Mask must be a 2D CUDA tensor");
@@ -487,6 +498,7 @@ Tensor gemm_dsd(const Tensor& A, const Tensor& B, const Tensor& mask, int64_t re
     py::gil_scoped_release no_gil;
     at::NoGradGuard no_grad;
     check_operand(A, "A");
+    check_mask_device(mask, A);
     c10::cuda::OptionalCUDAGuard guard(A.device());
     const Launch L(A.device());
     const Tensor plan = plan_from_mask(mask, A.size(0), A.size(1), rep_r, rep_c, L.stream);
@@ -502,6 +514,7 @@ Tensor gemm_sdd(const Tensor& A, const Tensor& B, const Tensor& mask, int64_t re
     at::NoGradGuard no_grad;
     check_operand(A, "A");
     check_operand(B, "B");
+    check_mask_device(mask, A);
     c10::cuda::OptionalCUDAGuard guard(A.device());
     const Launch L(A.device());
     const Tensor plan = plan_from_mask(mask, A.size(0), B.size(0), rep_r, rep_c, L.stream);
@@ -597,6 +610,7 @@ Tensor conv2d(const Tensor& input_, const Tensor& kernel_, const std::optional<T
     py::gil_scoped_release no_gil;
     if (!input_.is_cuda() || !kernel_.is_cuda()) bad("input and kernel must be CUDA");
     if (input_.device() != kernel_.device()) bad("input and kernel must be on the same device");
+    check_plan_device(plan_, input_.device());
     no_forward_ad("SparseDropConv2d", {input_, kernel_});
     const Tensor &input = input_, &kernel = kernel_;
     const bool amp = at::autocast::is_autocast_enabled(at::kCUDA);
