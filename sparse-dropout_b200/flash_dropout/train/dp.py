@@ -255,7 +255,7 @@ class _FusedAdamW:
     def _describe(self, optimizer) -> bool:
         self._native, self._seen = None, []
         seen, tensors, groups = [], [], []
-        device = optimizer.param_groups[0]["params"][0].device
+        device = next((p.device for g in optimizer.param_groups for p in g["params"]), None)      # (groups may be empty)
         for i, group in enumerate(optimizer.param_groups):
             for p in group["params"]:
                 st = optimizer.state.get(p)

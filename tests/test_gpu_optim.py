@@ -75,3 +75,21 @@ def test_a_model_that_has_been_stepped_is_freed(built_lib):
     del model, dp, opt
     gc.collect()
     assert all(r() is None for r in gone)
+
+
+@pytest.mark.parametrize("groups", [[[], [8]], [[8], []], [[], []]])
+def test_empty_groups(built_lib, groups):
+    """What a decay / no-decay split can leave behind is stepped as by the optimizer alone."""
+    from flash_dropout.train.dp import _FusedAdamW
+    sides = []
+    for ours in (False, True):
+        params = [[torch.nn.Parameter(torch.ones(n, device=DEV)) for n in ns] for ns in groups]
+        opt = torch.optim.AdamW([dict(params=ps) for ps in params], lr=0.1, fused=True)
+        fused = _FusedAdamW()
+        for k in range(3):
+            for p in sum(params, []):
+                p.grad = torch.full_like(p, k + 1.0) if p.grad is None else p.grad.fill_(k + 1.0)
+            fused.step(opt) if ours else opt.step()
+        sides.append(sum(params, []))
+    for a, b in zip(*sides):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-7)
