@@ -216,8 +216,9 @@ class _FusedAdamW:
 
     It updates the optimizer's own state tensors in place, so ``state_dict()``, checkpoints and a later ``optimizer.step()``
     see nothing unusual.  Anything the kernel does not do (AMSGrad, maximize, tensor learning rates, step counters on the
-    host, hooks, a patched ``step``, a gradient scaler, parameters without a gradient) and the first step, which creates
-    the state, are left to the optimizer itself.  The description of the tensors is made once and checked at every step."""
+    host, hooks, a patched ``step``, a gradient scaler, parameters without a gradient or without elements) and the first
+    step, which creates the state, are left to the optimizer itself.  The description of the tensors is made once and
+    checked at every step."""
 
     MAX_GROUPS = 8                                     # SD_ADAMW_MAX_GROUPS
 
@@ -259,7 +260,7 @@ class _FusedAdamW:
         for i, group in enumerate(optimizer.param_groups):
             for p in group["params"]:
                 st = optimizer.state.get(p)
-                if p.grad is None or not st or "step" not in st:
+                if p.grad is None or not p.numel() or not st or "step" not in st:
                     return False
                 entry = (p, p.grad, st["exp_avg"], st["exp_avg_sq"], st["step"])
                 if not all(isinstance(t, torch.Tensor) and t.layout == torch.strided and t.is_cuda and t.dtype == torch.float32

@@ -93,3 +93,16 @@ def test_empty_groups(built_lib, groups):
         sides.append(sum(params, []))
     for a, b in zip(*sides):
         torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("sizes", [[0, 8], [8, 0]])
+def test_parameters_without_elements(built_lib, sizes):
+    """The kernel's table has no place for them: the optimizer steps such a model by itself."""
+    from flash_dropout.train.dp import _FusedAdamW
+    params = [torch.nn.Parameter(torch.ones(n, device=DEV)) for n in sizes]
+    opt, fused = torch.optim.AdamW(params, lr=0.1, fused=True), _FusedAdamW()
+    for p in params:
+        p.grad = torch.ones_like(p)
+    for _ in range(3):
+        fused.step(opt)
+    assert fused._native is None and all(opt.state[p]["step"].item() == 3 for p in params)
