@@ -218,12 +218,15 @@ class _FusedAdamW:
     see nothing unusual.  Anything the kernel does not do (AMSGrad, maximize, tensor learning rates, step counters on the
     host, hooks, a patched ``step``, a gradient scaler, parameters without a gradient or without elements) and the first
     step, which creates the state, are left to the optimizer itself.  The description of the tensors is made once and
-    checked at every step."""
+    checked at every step.  Where none can be made (a gradient that is not 16-byte aligned, say) the next attempt waits for
+    1, 2, 4, ... 64 steps: it walks over every tensor in Python, for nothing."""
 
     MAX_GROUPS = 8                                     # SD_ADAMW_MAX_GROUPS
+    MAX_PAUSE = 64                                     # steps between two attempts to describe an optimizer
 
     def __init__(self):
         self._native = None
+        self._pause, self._wait = 1, 0                 # steps from the next failed attempt to the one after it; steps left
         self._seen: list = []                          # (parameter, gradient, state, exp_avg, exp_avg_sq, step)
 
     @staticmethod
@@ -278,12 +281,22 @@ class _FusedAdamW:
         self._seen = seen
         return True
 
+    def _try_to_describe(self, optimizer) -> bool:
+        if self._wait > 1:
+            self._wait -= 1
+            return False
+        if not torch.cuda.is_available() or torch.cuda.is_current_stream_capturing():
+            return False
+        done = self._describe(optimizer)
+        self._wait = 0 if done else self._pause
+        self._pause = 1 if done else min(2 * self._pause, self.MAX_PAUSE)
+        return done
+
     def step(self, optimizer) -> None:
         if self._plain(optimizer):
             if self._native is not None and not self._current(optimizer):
                 self._native = None
-            if self._native is not None or (torch.cuda.is_available() and not torch.cuda.is_current_stream_capturing()
-                                            and self._describe(optimizer)):
+            if self._native is not None or self._try_to_describe(optimizer):
                 hyper = []
                 for g in optimizer.param_groups:
                     hyper += (g["lr"], *g["betas"], g["eps"], g["weight_decay"])

@@ -17,3 +17,17 @@ def test_an_empty_first_group(monkeypatch):
         for _ in range(2):
             _FusedAdamW().step(opt)
     assert opt.state[p]["step"].item() == 2 and bool((p < 1).all())
+
+
+def test_an_optimizer_that_cannot_be_described_is_looked_at_ever_less_often(monkeypatch):
+    """The walk over its tensors is repeated after 1, 2, 4, ... 64 steps, and at once after it has been of use."""
+    from flash_dropout.train.dp import _FusedAdamW
+    p = torch.nn.Parameter(torch.ones(8))
+    p.grad = torch.ones(8)
+    opt, fused, looked = torch.optim.AdamW([p], lr=0.1), _FusedAdamW(), []
+    monkeypatch.setattr(fused, "_describe", lambda optimizer: looked.append(int(opt.state[p]["step"].item() if opt.state else 0)) or False)
+    with monkeypatch.context() as m:
+        _with_cuda(m)
+        for _ in range(260):
+            fused.step(opt)
+    assert looked == [0, 1, 3, 7, 15, 31, 63, 127, 191, 255] and opt.state[p]["step"].item() == 260
