@@ -52,3 +52,24 @@ def test_anything_else_is_torch(built_lib):
     (g,) = torch.autograd.grad(gelu(a).sum(), a, create_graph=True)
     g.sum().backward()
     assert a.grad is not None
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_no_result_is_further_off_than_torch(built_lib, dtype):
+    """Over all finite 16-bit inputs, value and derivative against fp64: never further than torch's own kernels."""
+    from flash_dropout.layers.gelu import GELU
+    x = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(dtype).to(DEV)
+    x = x[torch.isfinite(x)]
+    dy = torch.randn(x.numel(), generator=torch.Generator().manual_seed(1)).to(dtype).to(DEV)
+    exact = x.double().requires_grad_()
+    F.gelu(exact).backward(dy.double())
+    sides = []
+    for module in (GELU(), torch.nn.GELU()):
+        a = x.clone().requires_grad_()
+        y = module(a)
+        y.backward(dy)
+        sides.append((y.detach(), a.grad))
+    for ours, torchs, want in zip(*sides, (F.gelu(x.double()), exact.grad)):
+        inside = want.abs() < torch.finfo(dtype).max / 2
+        further = (ours.double() - want).abs() > (torchs.double() - want).abs()
+        assert not bool(further[inside].any()), f"{int(further[inside].sum())} of {x.numel()}"
