@@ -807,7 +807,10 @@ struct SparseDropGeluBackward : public Node {
     variable_list gradients(variable_list&& grads) {
         if (!grads[0].defined()) return {Tensor()};
         const Tensor h = x.unpack();
-        if (at::GradMode::is_enabled()) return {at::gelu_backward(grads[0], h)};     // the gradient's own graph is wanted
+        // the gradient's own graph is wanted, or it carries a batch dimension or a tangent that only torch's operators follow
+        if (at::GradMode::is_enabled() || at::isTensorSubclassLike(grads[0]) || at::isTensorSubclassLike(h) ||
+            torch::autograd::isFwGradDefined(grads[0]))
+            return {at::gelu_backward(grads[0], h)};
         Tensor dy = grads[0];
         if (dy.scalar_type() != h.scalar_type()) dy = dy.to(h.scalar_type());
         dy = dy.contiguous();

@@ -73,3 +73,21 @@ def test_no_result_is_further_off_than_torch(built_lib, dtype):
         inside = want.abs() < torch.finfo(dtype).max / 2
         further = (ours.double() - want).abs() > (torchs.double() - want).abs()
         assert not bool(further[inside].any()), f"{int(further[inside].sum())} of {x.numel()}"
+
+
+def test_batched_and_dual_gradients_are_torch(built_lib):
+    """A gradient that carries a batch dimension or a tangent of its own is differentiated by torch's operators."""
+    import torch.autograd.forward_ad as fwad
+    from flash_dropout.layers.gelu import GELU
+    x = torch.randn(64, 48, device=DEV).half().requires_grad_()
+    y = GELU()(x)
+    dys = torch.randn(3, 64, 48, device=DEV).half()
+    (got,) = torch.autograd.grad(y, x, dys, is_grads_batched=True, retain_graph=True)
+    for g, dy in zip(got, dys):
+        torch.testing.assert_close(g, torch.ops.aten.gelu_backward(dy, x.detach()))
+    with fwad.dual_level():
+        (g,) = torch.autograd.grad(y, x, fwad.make_dual(dys[0], dys[1]))
+        value, tangent = fwad.unpack_dual(g)
+    torch.testing.assert_close(value, torch.ops.aten.gelu_backward(dys[0], x.detach()))
+    assert tangent is not None
+    torch.testing.assert_close(tangent, torch.ops.aten.gelu_backward(dys[1], x.detach()))
