@@ -12,6 +12,8 @@
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAException.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -95,49 +97,93 @@ inline Tensor empty2(int64_t a, int64_t b, at::ScalarType t, const at::Device& d
 inline Tensor empty_bytes(int64_t n, const at::Device& d) { return at::detail::empty_cuda({n}, at::kByte, d, std::nullopt); }
 
 // ---------------------------------------------------------------- per-device state
-// The failure-detection words and the split-schedule workspaces, one per (device, stream) that has launched products:
-// launches that can overlap on the GPU must not share a workspace.  Lives until the process exits.
+// The failure-detection words of a device, and the split-schedule workspaces of the streams that have launched products on it:
+// launches that can overlap on the GPU must not share a workspace.  Live until the process exits.
+//
+// A CUDA graph has workspaces of its own: they come from its memory pool and are cleared by the graph itself, at every replay.
+// Only the last capture's are held on to here, for as long as the capture asks for them; the pool keeps their memory with the
+// graph.  One shared by the graphs captured on a stream would be cleared by the first of them only, and used by two replays
+// at once on different streams.
+struct Captured {
+    unsigned long long id = 0;
+    Tensor workspace;
+};
 struct DeviceState {
     Tensor status;
     std::unordered_map<cudaStream_t, Tensor> workspaces;
+    std::unordered_map<cudaStream_t, Captured> captured;
 };
 std::mutex& state_mutex() { static auto* m = new std::mutex; return *m; }
 std::unordered_map<int, DeviceState>& states() { static auto* s = new std::unordered_map<int, DeviceState>; return *s; }
 
+// Which capture the stream is in; 0: none.
+unsigned long long capture_of(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 Tensor status_tensor(int dev) {
     std::lock_guard<std::mutex> lock(state_mutex());
     DeviceState& s = states()[dev];
-    if (!s.status.defined())
-        s.status = at::zeros({4}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, c10::DeviceIndex(dev))));
+    if (s.status.defined()) return s.status;
+    const at::Device d(at::kCUDA, c10::DeviceIndex(dev));
+    const auto ints = at::TensorOptions().dtype(at::kInt).device(d);
+    if (!capture_of(c10::cuda::getCurrentCUDAStream(d.index()).stream())) {
+        s.status = at::zeros({4}, ints);
+        return s.status;
+    }
+    // The first launch of all is being captured.  The words outlive the graph, and must be zero before any replay of it.
+    c10::cuda::CUDAGuard guard(d);
+    c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    void* p = nullptr;
+    cudaStream_t own = nullptr;
+    C10_CUDA_CHECK(cudaMalloc(&p, 4 * sizeof(int)));
+    C10_CUDA_CHECK(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+    C10_CUDA_CHECK(cudaMemsetAsync(p, 0, 4 * sizeof(int), own));
+    C10_CUDA_CHECK(cudaStreamSynchronize(own));
+    C10_CUDA_CHECK(cudaStreamDestroy(own));
+    s.status = at::from_blob(p, {4}, ints);
     return s.status;
 }
 Tensor workspace_tensor(int dev, cudaStream_t stream) {
+    const unsigned long long capture = capture_of(stream);
     std::lock_guard<std::mutex> lock(state_mutex());
-    Tensor& ws = states()[dev].workspaces[stream];
-    if (!ws.defined()) {
+    DeviceState& s = states()[dev];
+    Captured* c = capture ? &s.captured[stream] : nullptr;
+    Tensor& ws = c ? c->workspace : s.workspaces[stream];
+    if (!ws.defined() || (c && c->id != capture)) {
         const at::Device d(at::kCUDA, c10::DeviceIndex(dev));
         c10::cuda::CUDAGuard guard(d);
         Tensor t = empty_bytes(int64_t(sd_workspace_bytes()), d);
         check_rc(sd_workspace_init(t.data_ptr(), stream));
         ws = t;
+        if (c) c->id = capture;
     }
     return ws;
 }
 
-// What every launch needs besides its operands.  The two pointers are looked up once per thread, device and stream.
+// What every launch needs besides its operands.  The two pointers are looked up once per thread, device, stream and capture.
 struct Launch {
     cudaStream_t stream;
     int* status;
     void* ws;
     explicit Launch(const at::Device& d) {
-        struct Cached { int dev = -1; cudaStream_t stream = nullptr; int* status = nullptr; void* ws = nullptr; };
+        struct Cached { int dev = -1; cudaStream_t stream = nullptr; unsigned long long capture = 0; int* status = nullptr; void* ws = nullptr; };
         static thread_local Cached c;
         stream = c10::cuda::getCurrentCUDAStream(d.index()).stream();
-        if (c.dev != d.index() || c.stream != stream) {
+        const unsigned long long capture = capture_of(stream);
+        if (c.dev != d.index() || c.stream != stream || c.capture != capture) {
+            c.dev = -1;                            // (nothing is cached if one of the two throws)
             c.status = status_tensor(d.index()).data_ptr<int>();
             c.ws = workspace_tensor(d.index(), stream).data_ptr();
             c.dev = d.index();
             c.stream = stream;
+            c.capture = capture;
         }
         status = c.status;
         ws = c.ws;

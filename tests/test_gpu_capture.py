@@ -71,3 +71,56 @@ def test_a_tensor_that_a_replay_writes(built_lib, operands):
     g.replay()
     y2 = _product(h, wb)
     _close(y2, h, wb)
+
+
+def _long(seed):
+    """Operands of a product that is cut along its reduction: two tiles, 32 K tiles."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return tuple((torch.randn(256, 4096, generator=g, device=DEV) * 4096 ** -0.25).half() for _ in range(2))
+
+
+def test_every_graph_has_a_workspace_of_its_own(built_lib):
+    """Cleared by its own replay, not by that of an earlier graph: the second one replays first."""
+    import flash_dropout
+    import flash_dropout.functional as F
+    from flash_dropout.cuda import binding_gemm as bg
+    graphs = []
+    for i in range(2):
+        x, w = _long(i)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            y = F.cuda_blockwise_dropout_matmul(x, w, 128, 0.0)
+            where = bg.workspace(DEV).data_ptr()
+            assert where == bg.workspace(DEV).data_ptr()
+        graphs.append((g, x, w, y, where))
+    assert graphs[0][4] != graphs[1][4]
+    for g, x, w, y, _ in (graphs[1], graphs[0], graphs[1]):
+        y.zero_()
+        g.replay()
+        torch.testing.assert_close(y.float(), x.float() @ w.float().T, rtol=2e-3, atol=2e-2)
+    flash_dropout.check_status(DEV)
+
+
+def test_the_status_word_of_a_first_launch_in_a_capture():
+    """In a process whose first launch is captured the word is zero before the first replay, and no replay clears it."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch, flash_dropout.functional as F
+from flash_dropout.cuda import binding_gemm as bg
+dev = torch.device("cuda:0")
+x = torch.ones(128, 128, device=dev, dtype=torch.float16)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    y = F.cuda_blockwise_dropout_matmul(x, x, 128, 0.0)
+word = bg.status_word(dev)
+assert word.tolist() == [0, 0, 0, 0], word.tolist()
+word[3] = 7
+g.replay()
+assert word.tolist() == [0, 0, 0, 7], word.tolist()
+assert bool((y == 128).all())
+"""
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sparse-dropout_b200")
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, env=dict(os.environ, PYTHONPATH=path))
