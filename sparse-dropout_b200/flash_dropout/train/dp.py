@@ -420,6 +420,8 @@ class GraphedTrainStep:
         with torch.cuda.graph(self.graph, capture_error_mode="thread_local"):
             self.loss = fwd_bwd()
         self._adamw_table = dp.adamw._native            # the captured update reads it at every replay
+        for p in dp._shadow_params:                     # what the capture recorded has not run: no copy is current
+            p._sd_w16 = None
 
     @staticmethod
     def _make_capturable(optimizer: torch.optim.Optimizer) -> bool:

@@ -124,3 +124,31 @@ assert bool((y == 128).all())
 """
     path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sparse-dropout_b200")
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300, env=dict(os.environ, PYTHONPATH=path))
+
+
+def test_weights_between_a_capture_and_its_first_replay(built_lib):
+    """A step that updates outside its graph: until the first replay the 16-bit copies that the graph makes are those of the
+    warm-up's last step, so an eager forward casts the weights itself."""
+    from flash_dropout import random as sd_random
+    from flash_dropout.train import BasicNet, FlatGradDataParallel, GraphedTrainStep
+    torch.manual_seed(0)
+    model = BasicNet(256, 1, 256, 10, dict(p=0.5, variant="blockwise[cuda]", block_size=128)).to(DEV)
+    x, y = torch.rand(256, 256, device=DEV), torch.randint(0, 10, (256,), device=DEV)
+    dp = FlatGradDataParallel(model, fuse_wgrad=True)
+    dp.shadow_min_layers = 1
+    opt = torch.optim.AdamW(model.parameters(), lr=1e-1)
+    sd_random.manual_seed(3, subsequence=0)
+    try:
+        GraphedTrainStep(model, dp, opt, lambda m, a, b: torch.nn.functional.cross_entropy(m(a).float(), b), (x, y),
+                         autocast_dtype=torch.bfloat16, whole_step=False)
+        outs = []
+        for copies in (True, False):
+            for p in dp._shadow_params:
+                p._sd_w16 = p._sd_w16 if copies else None
+            sd_random.device_counter(DEV).zero_()
+            with torch.autocast("cuda", dtype=torch.bfloat16):
+                outs.append(model(x).detach())
+        assert torch.equal(*outs)
+    finally:
+        sd_random.disable_device_counter()
+        sd_random.follow_torch_seed()
