@@ -206,6 +206,18 @@ Tensor operand(const Tensor& x) {
     return reinterpret_cast<uintptr_t>(y.data_ptr()) % 16 == 0 ? y : y.clone();
 }
 
+// A saved tensor that came back for backward.  Hooks (torch.autograd.graph.saved_tensors_hooks) may return any tensor: the
+// kernels take its memory as it is, so one of another type, device or shape is refused.  Its strides are the caller's matter.
+Tensor came_back(Tensor t, at::IntArrayRef sizes, at::ScalarType type, const at::Device& dev) {
+    if (t.scalar_type() != type || t.device() != dev || t.sizes() != sizes || t.layout() != at::kStrided)
+        bad("a saved tensor came back from its hooks with another type, device or shape");
+    return t;
+}
+Tensor dense16(const Tensor& t) {                  // contiguous, on a 16-byte boundary
+    const Tensor c = t.contiguous();
+    return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 ? c.clone() : c;
+}
+
 // ---------------------------------------------------------------- block plans
 // How the mask of one call comes about: a plan that exists, or a draw from (seed, offset), the offset optionally
 // advanced by a counter in device memory.
@@ -278,6 +290,8 @@ struct SparseDropLinearBackward : public Node {
     int64_t block_m = 0, block_k = 0;
     bool pair_block = false;
     int64_t M = 0, K = 0, N = 0;
+    at::ScalarType type = at::kHalf;               // of the saved tensors
+    at::Device dev = at::Device(at::kCUDA, 0);
     std::vector<int64_t> lead;                     // shape of an input that is not 2-D
     double p = 0, draw_p = 0;                      // of the scale, and of the draw
     bool x_f32 = false, w_f32 = false;             // the layer's own tensors are fp32: their gradients leave in fp32
@@ -296,18 +310,19 @@ struct SparseDropLinearBackward : public Node {
 variable_list SparseDropLinearBackward::apply(variable_list&& grads) { return backward_call([&] { return gradients(std::move(grads)); }); }
 variable_list SparseDropLinearBackward::gradients(variable_list&& grads) {
     at::NoGradGuard no_grad;
-    Tensor x16 = x.unpack();
-    const Tensor w16 = w.unpack();
-    if (x16.dim() != 2) x16 = x16.view({M, K});
-    const at::Device dev = x16.device();
     c10::cuda::OptionalCUDAGuard guard(dev);
+    Tensor x16 = x.unpack();
+    x16 = x16.dim() == 2 ? came_back(x16, {M, K}, type, dev) : came_back(x16, lead, type, dev).reshape({M, K});
+    x16 = operand(x16);
+    const Tensor w16 = operand(came_back(w.unpack(), {N, K}, type, dev));
+    if (opt.input_relu && x16.stride(1) != 1) x16 = dense16(x16);
     const Launch L(dev);
     const float scale = float(1.0 / (1.0 - p));
-    const int dt = dtype_code(x16.scalar_type());
+    const int dt = dtype_code(type);
     const Tensor pl = plan.defined() ? plan : draw_plan(draw, M, K, dev, L.stream);
     Tensor dy = grads[0].defined() ? grads[0] : at::zeros({M, N}, x16.options());     // (any rank: only the element count matters)
     if (dy.scalar_type() != x16.scalar_type()) dy = dy.to(x16.scalar_type());
-    if (opt.relu && !opt.premasked) dy = at::threshold_backward(dy, y.unpack(shared_from_this()), 0);
+    if (opt.relu && !opt.premasked) dy = at::threshold_backward(dy, came_back(y.unpack(shared_from_this()), dy.sizes(), type, dev), 0);
     dy = operand(dy.dim() == 2 ? dy : dy.reshape({M, N}));
     const Mat mdy = mat(dy), mx = mat(x16), mdyt = mat_t(dy), mxt = mat_t(x16), mwt = mat_t(w16);
     Tensor dx, dw;
@@ -458,6 +473,8 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     node->M = M;
     node->K = K;
     node->N = N;
+    node->type = xs.scalar_type();
+    node->dev = dev;
     node->p = p;
     if (input.dim() != 2) node->lead = input.sizes().vec();
     node->x_f32 = input.scalar_type() == at::kFloat;
@@ -592,6 +609,8 @@ struct SparseDropConv2dBackward : public Node {
     SavedVariable x, w2d, cols;
     Tensor plan;
     ConvGeometry g;
+    at::ScalarType t = at::kHalf;                  // of the saved tensors
+    at::Device dev = at::Device(at::kCUDA, 0);
     double p = 0;
     bool fused = false, has_cols = false, x_f32 = false, w_f32 = false;
 
@@ -604,11 +623,10 @@ struct SparseDropConv2dBackward : public Node {
     variable_list apply(variable_list&& grads) override { return backward_call([&] { return gradients(std::move(grads)); }); }
     variable_list gradients(variable_list&& grads) {
         at::NoGradGuard no_grad;
-        const Tensor x16 = x.unpack(), w = w2d.unpack();
-        const at::Device dev = x16.device();
         c10::cuda::OptionalCUDAGuard guard(dev);
+        const Tensor x16 = dense16(came_back(x.unpack(), {g.N, g.C, g.H, g.W}, t, dev));
+        const Tensor w = operand(came_back(w2d.unpack(), {g.Kog, g.Kg}, t, dev));
         const Launch L(dev);
-        const at::ScalarType t = x16.scalar_type();
         const int dt = dtype_code(t);
         const float scale = float(1.0 / (1.0 - p));
         Tensor dy = grads[0].defined() ? grads[0] : at::zeros({g.N, g.Ko, g.P, g.Q}, x16.options());
@@ -625,7 +643,8 @@ struct SparseDropConv2dBackward : public Node {
                 check_rc(sd_conv_dsd_dw(x16.data_ptr(), SD_CONV_GEOM(g), mdy.p, mdy.rs, mdy.cs, dw.data_ptr(), g.Kg, 1, g.Kog,
                                         plan.data_ptr(), scale, dt, L.ws, L.status, L.stream));
             else {
-                const Tensor col = has_cols ? cols.unpack() : im2col_panels(x16, g, plan, L.stream);
+                const Tensor col = has_cols ? dense16(came_back(cols.unpack(), {tiles_of(g.M), g.Kg, TILE}, t, dev))
+                                            : im2col_panels(x16, g, plan, L.stream);
                 check_rc(sd_gemm_dsd_panels(col.data_ptr(), g.M, g.Kg, mdy.p, mdy.cs, mdy.rs, dw.data_ptr(), 1, g.Kg, g.Kog,
                                             plan.data_ptr(), SD_PLAN_COLS, scale, dt, L.ws, L.status, L.stream));
             }
@@ -747,6 +766,8 @@ Tensor conv2d(const Tensor& input_, const Tensor& kernel_, const std::optional<T
     if (node->has_cols) node->cols = SavedVariable(cols, false);
     node->plan = plan;
     node->g = g;
+    node->t = t;
+    node->dev = dev;
     node->p = p;
     node->fused = fused;
     node->x_f32 = input.scalar_type() == at::kFloat;
@@ -774,11 +795,13 @@ struct SparseDropLayerNormBackward : public Node {
     variable_list apply(variable_list&& grads) override { return backward_call([&] { return gradients(std::move(grads)); }); }
     variable_list gradients(variable_list&& grads) {
         at::NoGradGuard no_grad;
-        const Tensor x2 = x.unpack(), g = weight.unpack();
-        const at::Device dev = x2.device();
+        Tensor x2 = x.unpack(), g = weight.unpack();
+        const at::Device dev = rstd.device();
         c10::cuda::OptionalCUDAGuard guard(dev);
+        const int64_t n = shape.back(), rows = rstd.numel();
+        x2 = dense16(came_back(x2, shape, at::kFloat, dev));
+        g = dense16(came_back(g, {n}, at::kFloat, dev));
         cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-        const int64_t n = shape.back(), rows = x2.numel() / n;
         Tensor dy = grads[0].defined() ? grads[0] : at::zeros(shape, x2.options());
         const at::ScalarType t = dy.scalar_type();
         if (t != at::kFloat && t != at::kHalf && t != at::kBFloat16) dy = dy.to(at::kFloat);
@@ -846,6 +869,7 @@ inline bool aligned16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.da
 
 struct SparseDropGeluBackward : public Node {
     SavedVariable x;
+    at::ScalarType type = at::kHalf;
 
     std::string name() const override { return "SparseDropGeluBackward"; }
     void release_variables() override { x.reset_data(); }
@@ -858,11 +882,10 @@ struct SparseDropGeluBackward : public Node {
             torch::autograd::isFwGradDefined(grads[0]))
             return {at::gelu_backward(grads[0], h)};
         Tensor dy = grads[0];
-        if (dy.scalar_type() != h.scalar_type()) dy = dy.to(h.scalar_type());
-        dy = dy.contiguous();
-        if (!aligned16(dy)) dy = dy.clone();
-        const Tensor hc = h.is_contiguous() && aligned16(h) ? h : h.clone(at::MemoryFormat::Contiguous);   // (a hook may unpack another layout)
-        const at::Device dev = hc.device();
+        const at::Device dev = dy.device();
+        const Tensor hc = dense16(came_back(h, dy.sizes(), type, dev));
+        if (dy.scalar_type() != type) dy = dy.to(type);
+        dy = dense16(dy);
         c10::cuda::OptionalCUDAGuard guard(dev);
         Tensor dx = at::detail::empty_cuda(hc.sizes(), hc.scalar_type(), dev, std::nullopt);
         check_rc(sd_gelu_bwd(dy.data_ptr(), hc.data_ptr(), dx.data_ptr(), hc.numel(), dtype_code(hc.scalar_type()),
@@ -886,6 +909,7 @@ std::optional<Tensor> gelu(const Tensor& x) {
     std::shared_ptr<SparseDropGeluBackward> node(new SparseDropGeluBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x));
     node->x = SavedVariable(x, false);
+    node->type = t;
     torch::autograd::set_history(y, node);
     return y;
 }
