@@ -278,7 +278,7 @@ struct PyCallback {
 
 struct Options {
     bool relu = false, input_relu = false, premasked = false;
-    Tensor wgrad;                                  // fp32 [out, in]: the weight gradient goes straight there
+    Tensor wgrad;                                  // [out, in], fp32 or the operands' type: the weight gradient goes straight there
     bool wgrad_acc = false;
     std::shared_ptr<PyCallback> notify;
 };
@@ -342,20 +342,19 @@ variable_list SparseDropLinearBackward::gradients(variable_list&& grads) {
                                  pl.data_ptr(), scale, dt, L.ws, L.status, L.stream));
     }
     // dW^T (K, N) = (keep o x)^T (K, M) . dy (M, N) * scale, stored straight into dW (N, K)
-    if (opt.wgrad.defined()) {
-        check_rc(sd_gemm_dsd_f32(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, opt.wgrad.data_ptr<float>(), opt.wgrad.stride(1),
-                                 opt.wgrad.stride(0), int(K), int(N), int(M), pl.data_ptr(), SD_PLAN_COLS, scale, dt,
-                                 int(opt.wgrad_acc), L.ws, L.status, L.stream));
-        if (opt.notify) (*opt.notify)();
-    } else if (task_should_compute_output(1)) {
-        dw = empty2(N, K, w_f32 ? at::kFloat : w16.scalar_type(), dev);
-        if (w_f32)
-            check_rc(sd_gemm_dsd_f32(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, dw.data_ptr<float>(), 1, K, int(K), int(N), int(M),
-                                     pl.data_ptr(), SD_PLAN_COLS, scale, dt, 0, L.ws, L.status, L.stream));
+    Tensor target = opt.wgrad;
+    if (!target.defined() && task_should_compute_output(1)) target = dw = empty2(N, K, w_f32 ? at::kFloat : type, dev);
+    if (target.defined()) {
+        const Mat out = mat_t(target);
+        if (target.scalar_type() == at::kFloat)
+            check_rc(sd_gemm_dsd_f32(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, static_cast<float*>(out.p), out.rs, out.cs, int(K),
+                                     int(N), int(M), pl.data_ptr(), SD_PLAN_COLS, scale, dt, int(opt.wgrad.defined() && opt.wgrad_acc),
+                                     L.ws, L.status, L.stream));
         else
-            check_rc(sd_gemm_dsd(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, dw.data_ptr(), 1, K, int(K), int(N), int(M),
+            check_rc(sd_gemm_dsd(mxt.p, mxt.rs, mxt.cs, mdyt.p, mdyt.rs, mdyt.cs, out.p, out.rs, out.cs, int(K), int(N), int(M),
                                  pl.data_ptr(), SD_PLAN_COLS, scale, dt, L.ws, L.status, L.stream));
     }
+    if (opt.wgrad.defined() && opt.notify) (*opt.notify)();
     return {dx, dw};
 }
 
@@ -419,9 +418,10 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
             ", " + std::to_string(w16.size(1)) + ")");
     if (opt.wgrad.defined()) {
         const Tensor& t = opt.wgrad;
-        if (t.dim() != 2 || t.size(0) != N || t.size(1) != K || t.device() != dev || t.scalar_type() != at::kFloat ||
-            !(t.stride(0) == 1 || t.stride(1) == 1))
-            bad("out has the wrong shape, device or strides");
+        if (t.dim() != 2 || t.size(0) != N || t.size(1) != K || t.device() != dev || !(t.stride(0) == 1 || t.stride(1) == 1) ||
+            (t.scalar_type() != at::kFloat && t.scalar_type() != x16.scalar_type()))
+            bad("out has the wrong shape, dtype, device or strides");
+        if (opt.wgrad_acc && t.scalar_type() != at::kFloat) bad("accumulate needs an fp32 out");
     }
     const bool needs_grad = torch::autograd::compute_requires_grad(input, weight);
     Tensor xs, ws, out, plan;

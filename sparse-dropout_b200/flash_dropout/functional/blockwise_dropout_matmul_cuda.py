@@ -68,9 +68,9 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
                       the gradient this layer returns is already the gradient of the ReLU's input;
       grad_premasked  with ``relu``: the incoming gradient already carries this layer's ReLU derivative (its only
                       consumer is a layer called with ``input_relu``), so backward does not apply it again;
-      wgrad           ``(fp32 tensor [out, in], accumulate, notify)``: the weight gradient is written (or added) in fp32
-                      straight into that tensor by the dW epilogue instead of being returned to autograd; ``notify()``
-                      is called afterwards;
+      wgrad           ``(tensor [out, in], accumulate, notify)``: the weight gradient is written (or, in fp32, added)
+                      straight into that tensor, fp32 or of the operands' type, by the dW epilogue instead of being
+                      returned to autograd; ``notify()`` is called afterwards;
       recompute_plan  keep only (seed, offset) of the mask between forward and backward and draw the plan again there
                       (one more plan launch per layer in backward; the plan buffer, 4 bytes per tile and list entry, is
                       not kept alive).  Applies to plans drawn from a host-side offset, a given one with the block size

@@ -349,3 +349,23 @@ def test_recompute_plan_redraws_the_plan_it_was_given(built_lib, drawn, called):
         outs.append((y.detach(), xa.grad, wa.grad))
     for a, b, name in zip(outs[0], outs[1], ("y", "dx", "dw")):
         assert torch.equal(a, b), name
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_weight_gradient_into_a_16_bit_target(built_lib, dtype, transposed):
+    """The target of the fused weight gradient may have the operands' type: what autograd would have got, bit for bit."""
+    import flash_dropout.functional as F
+    from flash_dropout.cuda.binding_gemm import BlockPlan
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x, w, dy = (torch.randn(*s, generator=g, device=DEV).to(dtype) for s in ((384, 520), (264, 520), (384, 264)))
+    plan = BlockPlan.from_seed(384, 520, 128, 0.5, 5, 2, DEV)
+    wa = w.clone().requires_grad_()
+    F.cuda_blockwise_dropout_matmul(x, wa, 128, 0.5, plan=plan).backward(dy)
+    target = torch.full((520, 264), 7.0, device=DEV, dtype=dtype).T if transposed else torch.full((264, 520), 7.0, device=DEV, dtype=dtype)
+    wb = w.clone().requires_grad_()
+    F.cuda_blockwise_dropout_matmul(x, wb, 128, 0.5, plan=plan, wgrad=(target, False, None)).backward(dy)
+    assert wb.grad is None and torch.equal(target, wa.grad)
+    for bad, accumulate in ((target, True), (target.to(torch.bfloat16 if dtype == torch.float16 else torch.float16), False)):
+        with pytest.raises(RuntimeError):
+            F.cuda_blockwise_dropout_matmul(x, wb, 128, 0.5, plan=plan, wgrad=(bad, accumulate, None))
