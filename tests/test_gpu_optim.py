@@ -106,3 +106,33 @@ def test_parameters_without_elements(built_lib, sizes):
     for _ in range(3):
         fused.step(opt)
     assert fused._native is None and all(opt.state[p]["step"].item() == 3 for p in params)
+
+
+def _one_step(p, g, m, v, t, lr, decay, b1=0.9, b2=0.999, eps=1e-8):
+    p = p * (1 - lr * decay)
+    m = b1 * m + (1 - b1) * g
+    v = b2 * v + (1 - b2) * g * g
+    return p - lr / (1 - b1 ** t) * m / (v.sqrt() / (1 - b2 ** t) ** 0.5 + eps), m, v
+
+
+@pytest.mark.parametrize("lr,decay", [(1e-3, 0.01), (1e-2, 0.0)])
+def test_an_update_is_as_precise_as_torchs(built_lib, lr, decay):
+    """Largest and rms error of one step against fp64 from the same state, over half a million elements; 5 % for the statistics
+    of rounding."""
+    from flash_dropout.train.dp import _FusedAdamW
+    errors = []
+    for ours in (False, True):
+        gen = torch.Generator(device=DEV).manual_seed(7)
+        p = torch.nn.Parameter(torch.randn(1 << 19, generator=gen, device=DEV) * 0.03)
+        p.grad = torch.zeros_like(p)
+        opt, fused = torch.optim.AdamW([p], lr=lr, weight_decay=decay, fused=True, capturable=True), _FusedAdamW()
+        for k in range(5):
+            p.grad.copy_(torch.randn(p.shape, generator=gen, device=DEV) * 10.0 ** -k)
+            st = opt.state[p]
+            before = [t.detach().double() for t in (p, p.grad, *(st.get(n, torch.zeros_like(p)) for n in ("exp_avg", "exp_avg_sq")))]
+            fused.step(opt) if ours else opt.step()
+        want = _one_step(*before, 5, lr, decay)
+        err = [(a.detach().double() - b).abs() for a, b in zip((p, st["exp_avg"], st["exp_avg_sq"]), want)]
+        errors.append([(e.max().item(), e.square().mean().sqrt().item()) for e in err])
+    for theirs, mine, name in zip(*errors, ("p", "exp_avg", "exp_avg_sq")):
+        assert all(b <= 1.05 * a for a, b in zip(theirs, mine)), (name, theirs, mine)
