@@ -107,12 +107,8 @@ def blockwise_dropout_conv2d(input: torch.Tensor, kernel: torch.Tensor, block_si
     through the kept-block im2col stage."""
     assert 0 <= p < 1, "Dropout probability must be in [0, 1)"
     if torch.jit.is_tracing():
-        return recorded(lambda x, k: _conv2d(x, k, block_size, p, padding, stride, dilation, plan, recompute_cols, fused), input,
-                        kernel)
-    return _conv2d(input, kernel, block_size, p, padding, stride, dilation, plan, recompute_cols, fused)
-
-
-def _conv2d(input, kernel, block_size, p, padding, stride, dilation, plan, recompute_cols, fused) -> torch.Tensor:
+        return recorded(blockwise_dropout_conv2d, (input, kernel), block_size, p, padding, stride, dilation, plan, recompute_cols,
+                        fused)
     if torch.is_autocast_enabled("cuda"):
         # fp32 tensors are cast inside the operator and get their gradients in fp32; others by autograd
         dt = torch.get_autocast_dtype("cuda")

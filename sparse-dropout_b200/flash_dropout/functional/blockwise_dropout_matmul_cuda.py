@@ -83,14 +83,8 @@ def blockwise_dropout_matmul(input: torch.Tensor, weight: torch.Tensor, block_si
     """
     assert 0 <= p < 1, "Dropout probability must be in [0, 1)"
     if torch.jit.is_tracing():
-        return recorded(lambda x, w: _matmul(x, w, block_size, p, plan, relu, input_relu, grad_premasked, wgrad,
-                                             recompute_plan, None, any_rank), input, weight)
-    return _matmul(input, weight, block_size, p, plan, relu, input_relu, grad_premasked, wgrad, recompute_plan, weight_lowp,
-                   any_rank)
-
-
-def _matmul(input, weight, block_size, p, plan, relu, input_relu, grad_premasked, wgrad, recompute_plan, weight_lowp,
-            any_rank) -> torch.Tensor:
+        return recorded(blockwise_dropout_matmul, (input, weight), block_size, p, plan, relu, input_relu, grad_premasked, wgrad,
+                        recompute_plan, None, any_rank)
     rep_r, rep_c = _rep(block_size)
     draw_p = p
     seed = offset = 0

@@ -13,7 +13,7 @@ class _Recorded(torch.autograd.Function):
     @staticmethod
     def forward(ctx, call, *tensors):
         state = torch._C._get_tracing_state()
-        torch._C._set_tracing_state(None)          # what the call does inside is not recorded
+        torch._C._set_tracing_state(None)          # the call itself is not recorded, and sees no trace
         try:
             with torch.enable_grad(), torch.autocast("cuda", enabled=False):
                 leaves = [t.detach().requires_grad_(needed) for t, needed in zip(tensors, ctx.needs_input_grad[1:])]
@@ -33,9 +33,9 @@ class _Recorded(torch.autograd.Function):
         return (None, *(next(grads) if t.requires_grad else None for t in ctx.leaves))
 
 
-def recorded(call, *tensors):
-    """``call(*tensors)`` as one operation of the trace that is being recorded.  Under autocast the tensors are cast here,
-    by operators that the trace sees."""
+def recorded(operator, tensors, *rest):
+    """``operator(*tensors, *rest)`` as one operation of the trace that is being recorded.  Under autocast the tensors are
+    cast here, by operators that the trace sees."""
     if torch.is_autocast_enabled("cuda"):
         tensors = [t.to(torch.get_autocast_dtype("cuda")) for t in tensors]
-    return _Recorded.apply(call, *tensors)
+    return _Recorded.apply(lambda *new: operator(*new, *rest), *tensors)
