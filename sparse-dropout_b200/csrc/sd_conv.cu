@@ -600,7 +600,8 @@ static int make_geom(ConvGeom* g, int N, int C, int H, int W, int R, int S, int 
         return fail(SD_ERR_INVALID_ARG, "conv sizes must be positive");
     if (stride_h <= 0 || stride_w <= 0 || dil_h <= 0 || dil_w <= 0 || pad_h < 0 || pad_w < 0)
         return fail(SD_ERR_INVALID_ARG, "stride and dilation must be positive, padding non-negative");
-    const long long over_h = H + 2ll * pad_h - (long long)dil_h * (R - 1) - 1, over_w = W + 2ll * pad_w - (long long)dil_w * (S - 1) - 1;
+    const long long over_h = H + 2ll * pad_h - (long long)dil_h * (R - 1) - 1;   // rows and columns the filter can move over
+    const long long over_w = W + 2ll * pad_w - (long long)dil_w * (S - 1) - 1;
     if (over_h < 0 || over_w < 0) return fail(SD_ERR_INVALID_ARG, "the filter does not fit the padded input");
     const long long P = over_h / stride_h + 1, Q = over_w / stride_w + 1;
     const long long M = N * P * Q, K = (long long)C * R * S;

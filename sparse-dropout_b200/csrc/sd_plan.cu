@@ -535,7 +535,7 @@ __device__ __forceinline__ void plan_bits_body(const PlanArgs& a) {
 // holds the whole mask, a row word per lane, so that offsets and column words come from shuffles and each warp writes the
 // lists of one row and of one column.  A launch of this size is nothing but latency: 6.5 -> 5.4 us for
 // 32 x 32 tiles, 5.3 -> 4.7 for 20 x 24, 4.2 -> 3.9 for 8 x 8 against plan_bits_kernel and its seven barriers (back to back in
-// a CUDA graph).// Same outputs as plan_kernel.
+// a CUDA graph).  Same outputs as plan_kernel.
 __device__ __forceinline__ void plan_small_body(const PlanArgs& a) {
     static_assert(kPlanThreads == 1024, "a warp per row, a warp per column");
     __shared__ unsigned keepmask[32];

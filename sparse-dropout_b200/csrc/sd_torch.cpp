@@ -173,7 +173,13 @@ struct Launch {
     int* status;
     void* ws;
     explicit Launch(const at::Device& d) {
-        struct Cached { int dev = -1; cudaStream_t stream = nullptr; unsigned long long capture = 0; int* status = nullptr; void* ws = nullptr; };
+        struct Cached {
+            int dev = -1;
+            cudaStream_t stream = nullptr;
+            unsigned long long capture = 0;
+            int* status = nullptr;
+            void* ws = nullptr;
+        };
         static thread_local Cached c;
         stream = c10::cuda::getCurrentCUDAStream(d.index()).stream();
         const unsigned long long capture = capture_of(stream);
@@ -278,7 +284,7 @@ struct PyCallback {
 
 struct Options {
     bool relu = false, input_relu = false, premasked = false;
-    Tensor wgrad;                                  // [out, in], fp32 or the operands' type: the weight gradient goes straight there
+    Tensor wgrad;                                  // [out, in], fp32 or the operands' type: takes the weight gradient
     bool wgrad_acc = false;
     std::shared_ptr<PyCallback> notify;
 };
@@ -384,7 +390,8 @@ Tensor linear(const Tensor& input_, const Tensor& weight_, const std::optional<T
     const at::Device dev = input_.device();
     const bool amp = at::autocast::is_autocast_enabled(at::kCUDA);
     const at::ScalarType amp_t = amp ? at::autocast::get_autocast_dtype(at::kCUDA) : at::kFloat;
-    const bool lowp = amp && weight_lowp && opt.wgrad.defined() && weight_lowp->scalar_type() == amp_t && weight_lowp->sizes() == weight_.sizes();
+    const bool lowp =
+        amp && weight_lowp && opt.wgrad.defined() && weight_lowp->scalar_type() == amp_t && weight_lowp->sizes() == weight_.sizes();
     if (lowp && weight_lowp->device() != dev) bad("A and B must be on the same device");
     check_plan_device(plan_, dev);
     c10::cuda::OptionalCUDAGuard guard(dev);

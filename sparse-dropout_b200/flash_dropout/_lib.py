@@ -1,8 +1,9 @@
 """ctypes binding of libsparsedrop.so (the C ABI declared in include/sparsedrop.h), and the torch extension on top of it.
 
-Both are built in-tree by ``csrc/build.sh`` into ``lib/`` next to this package.  There is no fallback: if the library is missing, or no CUDA device is present when a
-kernel is requested, the call raises.  ``lib()`` is the C ABI itself; ``ext()`` is ``sd_torch.so`` (``csrc/sd_torch.cpp``), the
-native host path of the operators: what runs between a Python entry point and the C ABI on every call.
+Both are built in-tree by ``csrc/build.sh`` into ``lib/`` next to this package.  There is no fallback: if the library is
+missing, or no CUDA device is present when a kernel is requested, the call raises.  ``lib()`` is the C ABI itself; ``ext()``
+is ``sd_torch.so`` (``csrc/sd_torch.cpp``), the native host path of the operators: what runs between a Python entry point and
+the C ABI on every call.
 """
 from __future__ import annotations
 
